@@ -79,14 +79,17 @@ def sigma_plan_desc(mode, nt, R, B, ms=None):
     d = {"mode": mode, "name": PLAN_NAMES[mode],
          ("alpha_pass_threads" if streams else "beta_singles_threads" if groups
           else "row_kernel_threads"): nt}
-    if groups and nt == 0:
+    if groups and nt == 1:
+        d["singles"] = "same-spin part in the hole-string products, Coulomb pass"
+    elif groups and nt == 0:
         d["beta_singles"] = "hole-string products"
     elif groups:
         d["beta_singles"] = "row stream on C^T"
     if mode == 0:
         d["staged_rows"] = R
     elif mode in (4, 5, 7):
-        d["product_engine"] = (f"tcgen05 3xTF32, {R}-column chunks" if R in (32, 64) else
+        d["product_engine"] = ("tcgen05 8-bit digit products, 48-column chunks" if R == 128 else
+                               f"tcgen05 3xTF32, {R}-column chunks" if R in (32, 64) else
                                f"{R} column threads")
     else:
         d["product_ctas_per_sm"] = R % 16

@@ -206,7 +206,9 @@ jci_status jci_sigma_device_noalloc(jci_space *s, const void *v, void *sigma,
  * the beta singles as a row stream on the transpose, then the product of
  * mode 1 (6) or of mode 5 (7)), threads per CTA of the row kernel (modes
  * 3-4: of the alpha pass; modes 6-7: of the beta-singles stream, or 0 for
- * the beta singles as products over (N-1)-electron hole strings), `rows`
+ * the beta singles as products over (N-1)-electron hole strings, or, mode 7
+ * with rows 128 and batch 5-7, 1 for the singles of both spins split between
+ * the hole-string products and a Coulomb pass), `rows`
  * (mode 0: alpha rows staged per pass; modes 1-3 and 6: product CTAs per
  * SM, 0 = as many as fit, plus 16 for the panel cut into 256-column blocks
  * gathered block by block, plus 32 for one panel per alpha row built and
@@ -216,8 +218,10 @@ jci_status jci_sigma_device_noalloc(jci_space *s, const void *v, void *sigma,
  * 5, 7: column threads of the fused
  * product, 8 (CUDA cores, 32-column chunks) or 16 (tensor cores, 64-column
  * chunks: FP64 mma.sync in FP64, 3xTF32 in FP32), or in FP32 32 / 64 (the
- * tcgen05 engine, 32- / 64-column chunks)), `batch` (modes 1, 2, 5: alpha strings per CTA of the
- * row kernel; modes 3-4: threads per CTA of the beta pass; modes 6-7: the
+ * tcgen05 engine, 32- / 64-column chunks), or 128 (8-bit digit products on
+ * the tcgen05 integer tensor cores, 48-column chunks, FP64 and FP32; at most
+ * 64 alpha singles and 127 pairs)), `batch` (modes 1, 2, 5: alpha strings
+ * per CTA of the row kernel; modes 3-4: threads per CTA of the beta pass; modes 6-7: the
  * group kernel variant, 1 or 2 columns per thread, or 3, 4: the group's
  * excitation targets split over 4 warps with 2 or 1 columns per lane, or
  * 5-7: the same-spin doubles as dense products over (N-2)-electron hole

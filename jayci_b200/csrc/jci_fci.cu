@@ -47,7 +47,8 @@ struct FciTables {
     FciSpin<double> d[2];
     FciSpin<float> f[2];
     size_t smem_max = 0;
-    int tuned_nt[2] = {0, 0}, tuned_R[2] = {0, 0};  // per precision (autotuned)
+    bool tuned[2] = {false, false};                 // per precision (autotuned)
+    int tuned_nt[2] = {0, 0}, tuned_R[2] = {0, 0};
     int tuned_mode[2] = {0, 0}, tuned_B[2] = {1, 1};
     float tuned_ms[2] = {0.f, 0.f};
     int mix_grid[2] = {0, 0};      // resident CTAs of k_sigma_mixed
@@ -79,6 +80,9 @@ struct FciTables {
     size_t hbytes[2] = {0, 0};
     void *pbuf[2] = {nullptr, nullptr};  // their E blocks, per precision
     size_t pbytes[2] = {0, 0};
+    I8Tables i8;                   // fused product on the integer tensor cores
+    int i8_state = 0;              // as prs_state
+    uint32_t *clist[2] = {nullptr, nullptr};  // singles of each spin for k_coulomb
 };
 
 bool fci_supported(const jci_space *s) {
@@ -136,6 +140,9 @@ void fci_free(DeviceState *d) {
     cudaFree(f->cp_gidx);
     cudaFree(f->pbuf[0]);
     cudaFree(f->pbuf[1]);
+    i8_tables_free(&f->i8);
+    cudaFree(f->clist[0]);
+    cudaFree(f->clist[1]);
     delete f;
     d->fci = nullptr;
 }
@@ -1223,6 +1230,7 @@ template <typename T>
 struct StreamArgs {
     int rows, len;                // output rows x row length
     int nd, ns;                   // doubles / singles of every row (ns = 0: none)
+    int add;                      // 1: Y += result, 0: Y = result
     const int *dJ;                // [double][row] source row
     const T *dH;                  // [double][row] value with phase
     const uint32_t *fs;           // [single][row] source row | sign << 31
@@ -1293,7 +1301,7 @@ __global__ void __launch_bounds__(ITEMS <= 8 ? 1024 : 512)
 #pragma unroll
     for (int it = 0; it < ITEMS; it++) {
         int i = c0 + tid + it * nt;
-        if (i < c1) yr[i] = acc[it];
+        if (i < c1) yr[i] = a.add ? yr[i] + acc[it] : acc[it];
     }
 }
 
@@ -1430,6 +1438,10 @@ jci_status fci_prepare(jci_space *s) {
         }
         if (f->prs[sp].jrow) {
             jci_status r = pair_fill(s, &f->prs[sp], st);
+            if (r) return r;
+        }
+        if (sp == 1 && f->i8_state == 1) {
+            jci_status r = i8_fill(&f->i8, d->m2, st);
             if (r) return r;
         }
         if (sp == 1 && f->hst.srow) {
@@ -1868,13 +1880,41 @@ static jci_status launch_mixed2(jci_space *s, const FciArgs<T> &fa, const T *v, 
 }
 
 // Product engines of the fused plans (4, 5, 7): tx = 8 or 16 column threads
-// of jci_fci_ab.cu, or 32 / 64 = the FP32 tcgen05 engine (jci_fci_tc.cu) with
-// chunks of that many columns.
+// of jci_fci_ab.cu, 32 / 64 = the FP32 tcgen05 engine (jci_fci_tc.cu) with
+// chunks of that many columns, or 128 = the digit products on the tcgen05
+// integer tensor cores (jci_fci_i8.cu).
 static bool is_tc_engine(int tx) { return tx == 32 || tx == 64; }
+constexpr int kI8Engine = 128;
 // Column threads whose entry lists an engine reads (chunks of 4 tx columns).
 static int ab_table_tx(int tx) { return is_tc_engine(tx) ? tx / 4 : tx; }
 
-static bool ab_plan_possible(const FciTables *f, int tx, size_t w) {
+// Tables of the integer engine, built and filled on first use (not while a
+// stream is being captured).
+static jci_status i8_tables(jci_space *s, cudaStream_t st) {
+    FciTables *f = s->dev->fci;
+    if (f->i8_state) return f->i8_state > 0 ? JCI_OK : JCI_ERR_SPACE;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    JCI_CUDA(cudaStreamIsCapturing(st, &cs));
+    if (cs != cudaStreamCaptureStatusNone) return JCI_ERR_STATE;
+    jci_status r = i8_tables_build(s, f->npair, &f->i8);
+    if (r == JCI_OK) r = i8_fill(&f->i8, s->dev->m2, st);
+    if (r == JCI_ERR_SPACE) f->i8_state = -1;
+    if (r == JCI_OK) f->i8_state = 1;
+    return r;
+}
+
+// Threads of the alpha-singles stream behind the integer engine.
+static int i8_stream_threads(const FciTables *f) {
+    for (int nt : {256, 128})
+        if (stream_ok(f->nb, nt)) return nt;
+    return 0;
+}
+
+static bool ab_plan_possible(jci_space *s, int tx, size_t w, cudaStream_t st) {
+    const FciTables *f = s->dev->fci;
+    if (tx == kI8Engine)
+        return i8_tables(s, st) == JCI_OK && i8_smem(f->i8, f->sa, w) <= f->smem_max &&
+               i8_stream_threads(f);
     const AbShape sh{f->nb, f->sa, f->sb, f->nelb, f->npair};
     if (is_tc_engine(tx)) return w == sizeof(float) && tc_possible(sh, tx, f->smem_max);
     return ab_possible(sh, tx, w, f->smem_max);
@@ -1897,12 +1937,29 @@ static jci_status ab_tables(jci_space *s, int tx, cudaStream_t st, AbTables **ou
     return JCI_OK;
 }
 
-// Fused product kernel (jci_fci_ab.cu) with tx column threads.
+// Fused product kernel (jci_fci_ab.cu) with tx column threads.  The integer
+// engine leaves the alpha singles of unchanged beta strings out: they come
+// from a row stream here unless the plan takes them elsewhere (singles = 0).
 template <typename T>
 static jci_status launch_ab(jci_space *s, const FciArgs<T> &fa, const T *v, T *o,
-                            cudaStream_t st, int tx) {
+                            cudaStream_t st, int tx, bool singles = true) {
     AbTables *t = nullptr;
     const bool tc = is_tc_engine(tx);
+    if (tx == kI8Engine) {
+        FciTables *f = s->dev->fci;
+        jci_status r = i8_tables(s, st);
+        if (!r) r = i8_scratch(&f->i8, sizeof(T));
+        if (r) return r;
+        if (singles) {
+            StreamArgs<T> al;
+            al.rows = fa.na; al.len = fa.nb; al.nd = 0; al.ns = fa.sa; al.add = 1;
+            al.dJ = nullptr; al.dH = nullptr; al.fs = fa.fsA; al.fp = fa.fpA; al.a1 = fa.a1A;
+            al.jc = fa.jB; al.hd = nullptr; al.skip = fa.skip;
+            if ((r = launch_stream<T>(al, i8_stream_threads(f), v, o, st))) return r;
+        }
+        const I8Input<T> in{fa.sa, fa.fsA, fa.fpA, fa.m2, fa.skip};
+        return i8_launch<T>(f->i8, in, s->dev->device, v, o, f->tc_status, st);
+    }
     jci_status r = ab_tables(s, ab_table_tx(tx), st, &t);
     if (r) return r;
     AbArgs<T> m;
@@ -2051,15 +2108,15 @@ static jci_status pair_scratch(jci_space *s, int items, cudaStream_t st, T **E) 
 // block under 1 GiB of E, 64-column blocks, widest under 4 GiB).
 template <typename T>
 static jci_status launch_group(jci_space *s, int sp, const T *hd, int add, const int *skip,
-                               int items, const T *x, T *y, cudaStream_t st) {
+                               int items, const T *x, T *y, cudaStream_t st, int singles = 0) {
     FciTables *f = s->dev->fci;
     if (items >= 5) {
         jci_status r = pair_tables(s, st);
         T *E = nullptr;
         if (!r) r = pair_scratch<T>(s, items, st, &E);
         if (r) return r;
-        return pair_launch<T>(f->prs[sp], sp == 0 ? f->nb : f->na, items, x, y, hd, add, skip, E,
-                              s->dev->device, st);
+        return pair_launch<T>(f->prs[sp], sp == 0 ? f->nb : f->na, items, singles, x, y, hd, add,
+                              skip, E, s->dev->device, st);
     }
     jci_status r = group_tables(s, st);
     if (r) return r;
@@ -2097,6 +2154,7 @@ static jci_status stream_scratch(FciTables *f, T **ct, T **tau) {
 // row jocc[pair][Ia] (hmatels_1x, action_util.c:210)
 template <typename T>
 static void stream_args(const FciArgs<T> &a, StreamArgs<T> &al, StreamArgs<T> &be) {
+    al.add = be.add = 0;
     al.rows = a.na; al.len = a.nb; al.nd = a.da; al.ns = 0;
     al.dJ = a.dJA; al.dH = a.dHA; al.fs = nullptr; al.fp = nullptr; al.a1 = nullptr;
     al.jc = nullptr; al.hd = a.hd; al.skip = a.skip;
@@ -2117,6 +2175,43 @@ static jci_status launch_transposes(const FciTables *f, const T *v, T *ct, T *o,
     return JCI_OK;
 }
 
+// Whether the singles can be split (threads = 1 of plan 7): their same-spin
+// part inside the hole-string products, their Coulomb part by k_coulomb; the
+// lists are built on first use (not while a stream is being captured).
+constexpr int kSplitSingles = 1;
+static jci_status coulomb_lists(jci_space *s, cudaStream_t st) {
+    FciTables *f = s->dev->fci;
+    if (!coulomb_possible(f->na, f->npair, f->smem_max) ||
+        !coulomb_possible(f->nb, f->npair, f->smem_max))
+        return JCI_ERR_SPACE;
+    for (int sp = 0; sp < 2; sp++) {
+        if (f->clist[sp]) continue;
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        JCI_CUDA(cudaStreamIsCapturing(st, &cs));
+        if (cs != cudaStreamCaptureStatusNone) return JCI_ERR_STATE;
+        const SpinTables &t = s->dev->t[sp];
+        jci_status r = coulomb_list_build(sp == 0 ? f->na : f->nb, sp == 0 ? f->sa : f->sb, t.fsing,
+                                          t.fspair, &f->clist[sp], st);
+        if (r) return r;
+    }
+    return JCI_OK;
+}
+
+// Coulomb part of the singles of spin sp: on C (rows of the other spin's
+// strings) for the beta singles, on C^T for the alpha singles.
+template <typename T>
+static jci_status launch_coulomb(jci_space *s, const FciArgs<T> &a, int sp, int add, const T *x,
+                                 T *y, cudaStream_t st) {
+    FciTables *f = s->dev->fci;
+    jci_status r = coulomb_lists(s, st);
+    if (r) return r;
+    if (sp == 1)
+        return coulomb_launch<T>(f->na, f->nb, f->sb, f->npair, f->clist[1], a.jA, x, y, add, a.skip,
+                                 s->dev->device, st);
+    return coulomb_launch<T>(f->nb, f->na, f->sa, f->npair, f->clist[0], a.jB, x, y, add, a.skip,
+                             s->dev->device, st);
+}
+
 // One full sigma of one vector with the given plan.
 // mode 0: k_sigma_fci with R staged alpha rows.
 // modes 1, 2, 5: k_sigma_rows (nt threads, B rows per CTA), then the product:
@@ -2129,7 +2224,9 @@ static jci_status launch_transposes(const FciTables *f, const T *v, T *ct, T *o,
 //   kernel variant B: 1 or 2 columns per thread, or 3, 4: the union split
 //   over 4 warps with 2 or 1 columns per lane), the beta singles as a row
 //   stream on C^T (nt threads), then the product of mode 3 (6) or of
-//   mode 4 (7).
+//   mode 4 (7).  Mode 7 with nt = 1 (integer engine, hole-string doubles):
+//   the singles of both spins split between the hole-string products and
+//   k_coulomb.
 template <typename T>
 static jci_status run_plan(jci_space *s, FciArgs<T> a, int mode, int nt, int R, int B,
                            const T *v, T *o, cudaStream_t st) {
@@ -2143,6 +2240,15 @@ static jci_status run_plan(jci_space *s, FciArgs<T> a, int mode, int nt, int R, 
         stream_args(a, al, be);
         be.nd = 0;  // the beta doubles come from the group kernel
         if ((r = launch_transposes<T>(f, v, ct, o, tau, false, a.skip, st))) return r;
+        if (nt == kSplitSingles) {
+            // the diagonal, the largest term, last
+            if ((r = launch_coulomb<T>(s, a, 1, 0, v, o, st))) return r;
+            if ((r = launch_ab<T>(s, a, v, o, st, R, false))) return r;
+            if ((r = launch_coulomb<T>(s, a, 0, 0, ct, tau, st))) return r;
+            if ((r = launch_group<T>(s, 1, nullptr, 1, a.skip, B, ct, tau, st, 1))) return r;
+            if ((r = launch_transposes<T>(f, v, ct, o, tau, true, a.skip, st))) return r;
+            return launch_group<T>(s, 0, a.hd, 1, a.skip, B, v, o, st, 1);
+        }
         if ((r = nt == 0 ? launch_hs<T>(s, be, ct, tau, st) : launch_stream<T>(be, nt, ct, tau, st)))
             return r;
         if ((r = launch_group<T>(s, 1, nullptr, 1, a.skip, B, ct, tau, st))) return r;
@@ -2226,9 +2332,38 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
         int items = (f->nb + nt - 1) / nt;
         return !(nt > 32 * ((f->nb + 31) / 32) && nt > 128) && items <= 32;  // idle threads
     };
+    // the components of a plan are timed one by one; its best configuration is
+    // timed end to end before choosing
+    auto best_of = [&](auto fn) {
+        float m = 1e30f;
+        for (int k = 0; k < 3; k++) {
+            m = std::min(m, timeit(fn));
+            if (m > 50.f && m < 1e29f) break;  // as in timeit
+        }
+        return m;
+    };
+    // mode 7 with the integer product and the singles split, end to end
+    float bests = 1e30f;
+    int bsB = 5;
+    if (ab_plan_possible(s, kI8Engine, w, st) && coulomb_lists(s, st) == JCI_OK &&
+        group_possible(f) && pair_tables(s, st) == JCI_OK) {
+        for (int B : {5, 7}) {
+            const float ms =
+                best_of([&] { return run_plan<T>(s, a, 7, kSplitSingles, kI8Engine, B, v, o, st); });
+            if (ms < bests) { bests = ms; bsB = B; }
+        }
+        if (err) cudaGetLastError();
+        err = JCI_OK;  // a space too large for its scratch just drops the plan
+    }
+    // From 2^21 determinants on it beats every other plan (FP64, against the
+    // best of the others: 1.60 to 1.85 ms at 2.9 M determinants, 6.8 to 12.4 at
+    // 11.8 M, 123 to 232 at 165.6 M; below, at 0.85 M, they lie within a few
+    // percent), and timing those would take half a minute at the largest.
+    const bool only_split = bests < 1e30f && n >= (1ll << 21);
     // mode 0: one kernel, R staged rows
     float best0 = 1e30f;
     int b0nt = 0, b0R = 0;
+    if (!only_split)
     for (int nt : nts) {
         int items = (f->nb + nt - 1) / nt;
         if (!useful(nt) || (nt == 1024 && items > 2)) continue;
@@ -2246,19 +2381,19 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
     ar.R = 0;
     float bpanel = 1e30f, bmix2 = 1e30f, bab = 1e30f;
     int Rpanel = 1, Rmix2 = 1, txab = 0;
-    if (mixed_possible(f, w))
+    if (mixed_possible(f, w) && !only_split)
         // whole-row panel per CTA, column-blocked, row panels shared by all CTAs
         for (int R : {1, 2, 4, 16 + 1, 16 + 2, 16 + 4, 64 + 1, 64 + 2, 64 + 4}) {
             float ms = timeit([&] { return launch_mixed<T>(s, ar, v, o, st, R); });
             if (ms < bpanel) { bpanel = ms; Rpanel = R; }
         }
-    if (mixed2_possible(f, w))
+    if (mixed2_possible(f, w) && !only_split)
         for (int R : {1, 2}) {
             float ms = timeit([&] { return launch_mixed2<T>(s, ar, v, o, st, R); });
             if (ms < bmix2) { bmix2 = ms; Rmix2 = R; }
         }
-    for (int tx : {8, 16, 32, 64}) {
-        if (!ab_plan_possible(f, tx, w)) continue;
+    for (int tx : {8, 16, 32, 64, kI8Engine}) {
+        if (only_split || !ab_plan_possible(s, tx, w, st)) continue;
         float ms = timeit([&] { return launch_ab<T>(s, ar, v, o, st, tx); });
         if (ms < bab) { bab = ms; txab = tx; }
     }
@@ -2351,16 +2486,6 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
         err = JCI_OK;  // a space the group tables cannot hold just drops the plan
     }
     const int gmode = sab ? 7 : 6;
-    // the components were timed one by one; time each plan's best
-    // configuration end to end before choosing
-    auto best_of = [&](auto fn) {
-        float m = 1e30f;
-        for (int k = 0; k < 3; k++) {
-            m = std::min(m, timeit(fn));
-            if (m > 50.f && m < 1e29f) break;  // as in timeit
-        }
-        return m;
-    };
     if (b0nt) best0 = best_of([&] { return run_plan<T>(s, a, 0, b0nt, b0R, 1, v, o, st); });
     if (b1nt)
         best1 = best_of([&] { return run_plan<T>(s, a, b1mode, b1nt, b1R, b1B, v, o, st); });
@@ -2381,16 +2506,25 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
     cudaFree(v);
     cudaFree(o);
     if (err) return err;
-    if (!b0nt && !b1nt && !(b3a && b3b) && best6 >= 1e30f) return JCI_ERR_SPACE;
+    if (!b0nt && !b1nt && !(b3a && b3b) && best6 >= 1e30f && bests >= 1e30f)
+        return JCI_ERR_SPACE;
     int mode = 0;
     float best = best0;
     if (b1nt && best1 < best) { mode = b1mode; best = best1; }
     if (b3a && b3b && best3 < best) { mode = smode; best = best3; }
     if (best6 < best) { mode = gmode; best = best6; }
+    const bool split = bests < best;
+    if (split) {
+        mode = 7;
+        best = bests;
+        b6s = kSplitSingles;
+        b6i = bsB;
+    }
     const bool streams = mode == 3 || mode == 4, groups = mode == 6 || mode == 7;
+    f->tuned[prec] = true;
     f->tuned_mode[prec] = mode;
     f->tuned_nt[prec] = groups ? b6s : streams ? b3a : mode ? b1nt : b0nt;
-    f->tuned_R[prec] = (streams || groups) ? sR : mode ? b1R : b0R;
+    f->tuned_R[prec] = split ? kI8Engine : (streams || groups) ? sR : mode ? b1R : b0R;
     f->tuned_B[prec] = groups ? b6i : streams ? b3b : mode ? b1B : 1;
     f->tuned_ms[prec] = best;
     // drop the group tables unless a precision uses them
@@ -2398,6 +2532,11 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
     if (!groups && other != 6 && other != 7) {
         group_tables_free(&f->grp[0]);
         group_tables_free(&f->grp[1]);
+    }
+    const int eng = mode == 4 || mode == 5 || mode == 7 ? f->tuned_R[prec] : 0;
+    if (eng != kI8Engine && f->i8.scratch[prec]) {  // the integer engine's digits are not needed
+        cudaFree(f->i8.scratch[prec]);
+        f->i8.scratch[prec] = nullptr;
     }
     if (mode != 1 && mode != 3 && mode != 6 && f->tbuf[prec]) {  // the product panels are not needed
         cudaFree(f->tbuf[prec]);
@@ -2448,7 +2587,7 @@ static jci_status launch_fci(jci_space *s, int nvec, const T *V, T *S, long long
         a.dHA = (const T *)f->f[0].dblH; a.dHB = (const T *)f->f[1].dblH;
         a.hd = (const T *)d->hdf; a.m2 = (const T *)d->m2f;
     }
-    if (f->tuned_nt[prec] == 0) {
+    if (!f->tuned[prec]) {
         jci_status r = autotune<T>(s, a, st);
         if (r) return r;
     }
@@ -2479,20 +2618,25 @@ jci_status fci_force_plan(jci_space *s, int precision, int mode, int nt, int R, 
     int p = precision == JCI_FP32 ? 1 : 0;
     size_t w = p ? sizeof(float) : sizeof(double);
     if (mode == 6 || mode == 7) {
-        bool ok = mode == 6 ? mixed_possible(f, w) && R >= 0 : ab_plan_possible(f, R, w);
-        const bool beta_ok = nt == 0 ? hs_tables(s, s->dev->stream) == JCI_OK
+        bool ok = mode == 6 ? mixed_possible(f, w) && R >= 0 : ab_plan_possible(s, R, w, s->dev->stream);
+        bool ok1 = true;
+        if (nt == kSplitSingles)
+            ok1 = mode == 7 && R == kI8Engine && B >= 5 && coulomb_lists(s, s->dev->stream) == JCI_OK;
+        if (!ok1) return JCI_ERR_ARG;
+        const bool beta_ok = nt == kSplitSingles ? true
+                             : nt == 0 ? hs_tables(s, s->dev->stream) == JCI_OK
                                      : stream_ok(f->na, nt) && stream_smem(0, f->sb, w) <= f->smem_max;
         if (!ok || !group_possible(f) || !beta_ok || B < 1 || B > 7) return JCI_ERR_ARG;
         if (B >= 5 && pair_tables(s, s->dev->stream) != JCI_OK) return JCI_ERR_ARG;
     } else if (mode == 3 || mode == 4) {
-        bool ok = mode == 3 ? mixed_possible(f, w) && R >= 0 : ab_plan_possible(f, R, w);
+        bool ok = mode == 3 ? mixed_possible(f, w) && R >= 0 : ab_plan_possible(s, R, w, s->dev->stream);
         if (!ok || !stream_ok(f->nb, nt) || !stream_ok(f->na, B) ||
             stream_smem(f->da, 0, w) > f->smem_max || stream_smem(f->db, f->sb, w) > f->smem_max)
             return JCI_ERR_ARG;
     } else if (mode == 1 || mode == 2 || mode == 5) {
         bool ok = mode == 1   ? mixed_possible(f, w) && R >= 0
                   : mode == 2 ? mixed2_possible(f, w) && R >= 0
-                              : ab_plan_possible(f, R, w);
+                              : ab_plan_possible(s, R, w, s->dev->stream);
         if (!ok || !rows_ok(f->nb, nt, B) || rows_smem(f->nb, f->npair, f->da, B, w) > f->smem_max)
             return JCI_ERR_ARG;
     } else {
@@ -2504,7 +2648,8 @@ jci_status fci_force_plan(jci_space *s, int precision, int mode, int nt, int R, 
     }
     if (mode == 4 || mode == 5 || mode == 7) {  // tables are built here, outside any capture
         AbTables *t = nullptr;
-        jci_status r = ab_tables(s, ab_table_tx(R), s->dev->stream, &t);
+        jci_status r = R == kI8Engine ? i8_scratch(&f->i8, w)
+                                      : ab_tables(s, ab_table_tx(R), s->dev->stream, &t);
         if (r) return r;
     }
     if (mode == 6 || mode == 7) {
@@ -2522,6 +2667,7 @@ jci_status fci_force_plan(jci_space *s, int precision, int mode, int nt, int R, 
         jci_status r = ab_tables(s, kMixBlock / 4, s->dev->stream, &t);
         if (r) return r;
     }
+    f->tuned[p] = true;
     f->tuned_mode[p] = mode;
     f->tuned_nt[p] = nt;
     f->tuned_R[p] = R;

@@ -190,6 +190,133 @@ __global__ void __launch_bounds__(kPairThreads)
     }
 }
 
+// Phase 1 for hole strings with NF <= 10 free orbitals, on the FP64 tensor
+// cores in both precisions (FP32 operands are widened, so its sums are exact
+// to FP64 and half of the FMA form's time).  W_K is the same for every column,
+// so a warp keeps its fragments of the whole matrix in registers (72 doubles
+// a lane for 45 pairs) and the inner loop loads only X: 2 loads for 2 MT
+// MMAs, where reading W_K from shared memory bound the 16-row tiles above.
+// Rows are padded to 8 and k to 4, not to 16: 36 pairs (FCI(14,14)) take
+// 40 x 36 instead of 48 x 48.
+// Warp w owns columns 16 w .. + 15 of a 64-column chunk; the chunks of the
+// CTA's column segment are double-buffered with cp.async (16-byte pieces when
+// the rows allow them).
+// Measured, one spin's pass: FCI(14,14) FP64 1.23 -> 0.78 ms (FP64 tensor pipe
+// 75% busy), FP32 1.49 -> 0.74; FCI(16,16) FP64 19.6 -> 20.7 ms (two CTAs an
+// SM; X is streamed from DRAM), FP32 22.0 -> 21.9.
+constexpr int kMmaThreads = 128;
+template <typename T>
+__host__ __device__ constexpr int mma_ds() { return kPairCols + (sizeof(T) == 8 ? 4 : 8); }
+
+template <typename T, int NF>
+__global__ void __launch_bounds__(kMmaThreads, NF >= 10 ? 2 : 3)
+    k_pairs_mma(PairArgs<T> a, const T *__restrict__ X, T *__restrict__ E, int c0, int cb, int seg,
+                int vec) {
+    if (a.skip && *a.skip) return;
+    constexpr int NP = NF * (NF - 1) / 2, MT = (NP + 7) / 8, KS = (NP + 3) / 4;
+    constexpr int DS = mma_ds<T>();
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T *Ds = reinterpret_cast<T *>(smem_raw);                       // [2][4 KS][DS]
+    int *jr = reinterpret_cast<int *>(Ds + 2 * (size_t)4 * KS * DS);  // [NP]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int K = blockIdx.x;
+    const long long kb = (long long)K * NP;
+    for (int p = tid; p < NP; p += kMmaThreads) jr[p] = a.jrow[kb + p];
+    // rows of k past the pairs stay zero
+    for (int i = tid; i < (4 * KS - NP) * DS; i += kMmaThreads)
+        Ds[NP * DS + i] = Ds[(4 * KS + NP) * DS + i] = T(0);
+    __syncthreads();
+    const int cs = c0 + blockIdx.y * seg, c1 = min(min(a.len, c0 + cb), cs + seg);
+    constexpr int VE = 16 / sizeof(T);
+    auto stage = [&](int c, T *buf) {
+        if (vec) {
+            for (int idx = tid; idx < NP * (kPairCols / VE); idx += kMmaThreads) {
+                const int q = idx / (kPairCols / VE), cc = VE * (idx % (kPairCols / VE));
+                T *dst = buf + q * DS + cc;
+                if (c + cc < c1)  // c1 is a multiple of VE, or the row's end is
+                    __pipeline_memcpy_async(
+                        dst, X + (long long)(jr[q] & 0x7fffffff) * a.len + c + cc, 16);
+            }
+        } else {
+            for (int idx = tid; idx < NP * kPairCols; idx += kMmaThreads) {
+                const int q = idx / kPairCols, cc = idx % kPairCols;
+                if (c + cc < c1)
+                    __pipeline_memcpy_async(
+                        buf + q * DS + cc,
+                        X + (long long)(jr[q] & 0x7fffffff) * a.len + c + cc, sizeof(T));
+            }
+        }
+        __pipeline_commit();
+    };
+    const int nchunk = (c1 - cs + kPairCols - 1) / kPairCols;
+    if (nchunk > 0) stage(cs, Ds);
+    // this lane's elements of W_K: row 8 i + g, column 4 k + t
+    double w[MT][KS];
+#pragma unroll
+    for (int i = 0; i < MT; i++) {
+        const int p = 8 * i + g;
+        const size_t wr = p < NP ? (size_t)a.gp[kb + p] * a.ngp : 0;
+        const int jp = p < NP ? jr[p] : 0;
+#pragma unroll
+        for (int k = 0; k < KS; k++) {
+            const int q = 4 * k + t;
+            double v = 0.0;
+            if (p < NP && q < NP) {
+                v = (double)a.W[wr + a.gp[kb + q]];
+                if ((jp ^ jr[q]) < 0) v = -v;  // phi_p phi_q
+            }
+            w[i][k] = v;
+        }
+    }
+    for (int ci = 0; ci < nchunk; ci++) {
+        const int c = cs + ci * kPairCols;
+        const T *Dc = Ds + (size_t)(ci & 1) * 4 * KS * DS;
+        if (ci + 1 < nchunk) {
+            stage(c + kPairCols, Ds + (size_t)((ci + 1) & 1) * 4 * KS * DS);
+            __pipeline_wait_prior(1);
+        } else {
+            __pipeline_wait_prior(0);
+        }
+        __syncthreads();
+        double acc[MT][2][2];
+#pragma unroll
+        for (int i = 0; i < MT; i++)
+#pragma unroll
+            for (int n = 0; n < 2; n++) acc[i][n][0] = acc[i][n][1] = 0.0;
+        const T *bp = Dc + t * DS + 16 * warp + g;
+#pragma unroll
+        for (int k = 0; k < KS; k++) {
+            const double b0 = (double)bp[4 * k * DS], b1 = (double)bp[4 * k * DS + 8];
+#pragma unroll
+            for (int i = 0; i < MT; i++) {
+                pair_dmma(acc[i][0], w[i][k], b0);
+                pair_dmma(acc[i][1], w[i][k], b1);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < MT; i++) {
+            const int p = 8 * i + g;
+            if (p >= NP) continue;
+#pragma unroll
+            for (int n = 0; n < 2; n++) {
+                const int col = c + 16 * warp + 8 * n + 2 * t;
+                T *dst = E + (size_t)(kb + p) * cb + (col - c0);
+                if (col + 1 < c1) {
+                    if constexpr (sizeof(T) == 8)
+                        __stcs(reinterpret_cast<double2 *>(dst),
+                               make_double2(acc[i][n][0], acc[i][n][1]));
+                    else
+                        __stcs(reinterpret_cast<float2 *>(dst),
+                               make_float2((float)acc[i][n][0], (float)acc[i][n][1]));
+                } else if (col < c1) {
+                    dst[0] = (T)acc[i][n][0];
+                }
+            }
+        }
+        __syncthreads();
+    }
+}
+
 // Phase 2: Y[I][c] = sum_t E[pull[I][t]][c - c0] (+ hd X, + Y) for the
 // strings I of CTA row block blockIdx.x and the columns c0 + 256 blockIdx.y + tid.
 template <typename T>
@@ -226,15 +353,30 @@ __global__ void __launch_bounds__(kPairThreads)
 
 template <typename T>
 using PairKernel = void (*)(PairArgs<T>, const T *, T *, int, int);
+template <typename T>
+using MmaKernel = void (*)(PairArgs<T>, const T *, T *, int, int, int, int);
 
+// The form for wide hole strings (55, 66 and 78 pairs).
 template <typename T>
 PairKernel<T> pair_kernel(int RT) {
     switch (RT) {
-        case 1: return k_pairs_product<T, 1>;
-        case 2: return k_pairs_product<T, 2>;
-        case 3: return k_pairs_product<T, 3>;
         case 4: return k_pairs_product<T, 4>;
         case 5: return k_pairs_product<T, 5>;
+        default: return nullptr;
+    }
+}
+
+template <typename T>
+MmaKernel<T> mma_kernel(int nf) {
+    switch (nf) {
+        case 3: return k_pairs_mma<T, 3>;
+        case 4: return k_pairs_mma<T, 4>;
+        case 5: return k_pairs_mma<T, 5>;
+        case 6: return k_pairs_mma<T, 6>;
+        case 7: return k_pairs_mma<T, 7>;
+        case 8: return k_pairs_mma<T, 8>;
+        case 9: return k_pairs_mma<T, 9>;
+        case 10: return k_pairs_mma<T, 10>;
         default: return nullptr;
     }
 }
@@ -431,13 +573,14 @@ jci_status pair_tables_build(const jci_space *s, int spin, PairTables *t) {
                 pull[(size_t)i * nt + t2] = it->second * np + p;
             }
     }
+    t->nf = nf; t->fixed = fixed; t->nv = nv;
     t->nk = (int)nk; t->np = np; t->NP = NP; t->nt = nt; t->ngp = ngp; t->rows = ns;
     t->orb = orb;
     JCI_CUDA(cudaMalloc(&t->jrow, jrow.size() * sizeof(int)));
     JCI_CUDA(cudaMalloc(&t->gp, gp.size() * sizeof(uint16_t)));
     JCI_CUDA(cudaMalloc(&t->pull, pull.size() * sizeof(int)));
-    JCI_CUDA(cudaMalloc(&t->W64, (size_t)ngp * ngp * sizeof(double)));
-    JCI_CUDA(cudaMalloc(&t->W32, (size_t)ngp * ngp * sizeof(float)));
+    JCI_CUDA(cudaMalloc(&t->W64, 2 * (size_t)ngp * ngp * sizeof(double)));
+    JCI_CUDA(cudaMalloc(&t->W32, 2 * (size_t)ngp * ngp * sizeof(float)));
     JCI_CUDA(cudaMemcpy(t->jrow, jrow.data(), jrow.size() * sizeof(int), cudaMemcpyHostToDevice));
     JCI_CUDA(cudaMemcpy(t->gp, gp.data(), gp.size() * sizeof(uint16_t), cudaMemcpyHostToDevice));
     JCI_CUDA(cudaMemcpy(t->pull, pull.data(), pull.size() * sizeof(int), cudaMemcpyHostToDevice));
@@ -446,7 +589,12 @@ jci_status pair_tables_build(const jci_space *s, int spin, PairTables *t) {
 
 // W over the orbital pairs from the current integrals (the host copy that
 // the device integrals are made from): W[(ij)][(kl)] = (ik|jl) - (il|jk),
-// zero when the pairs share an orbital.
+// zero when the pairs share an orbital; behind it the same matrix with the
+// pairs that share one orbital filled in, which carries the same-spin part of
+// the singles too: a single k <- l of a string has one hole string K for each
+// of its other nv - 1 varying electrons m, with the element
+//   (kl|mm) - (km|ml) + h'_kl / (nv - 1),
+// h' the one-electron matrix with the orbitals common to every string.
 jci_status pair_fill(const jci_space *s, PairTables *t, cudaStream_t st) {
     const int no = (int)t->orb.size(), ngp = t->ngp;
     std::vector<int> pa(ngp), pb(ngp);
@@ -455,17 +603,34 @@ jci_status pair_fill(const jci_space *s, PairTables *t, cudaStream_t st) {
             pa[P] = t->orb[a];
             pb[P] = t->orb[b];
         }
-    t->w64.assign((size_t)ngp * ngp, 0.0);
-    t->w32.assign((size_t)ngp * ngp, 0.f);
-    const double *m2 = s->m2.data();
+    const size_t nw = (size_t)ngp * ngp;
+    t->w64.assign(2 * nw, 0.0);
+    t->w32.assign(2 * nw, 0.f);
+    const double *m1 = s->m1.data(), *m2 = s->m2.data();
+    auto h1 = [&](int k, int l) {
+        double v = m1[pair_index(k, l)];
+        for (int f : t->fixed)
+            v += m2[eri_index(pair_index(f, f), pair_index(k, l))] -
+                 m2[eri_index(pair_index(f, k), pair_index(f, l))];
+        return v / (t->nv - 1);
+    };
     for (int P = 0; P < ngp; P++)
         for (int Q = 0; Q < ngp; Q++) {
+            if (P == Q) continue;
             const int i = pa[P], j = pb[P], k = pa[Q], l = pb[Q];
-            if (i == k || i == l || j == k || j == l) continue;
-            const double w = m2[eri_index(pair_index(i, k), pair_index(j, l))] -
-                             m2[eri_index(pair_index(i, l), pair_index(j, k))];
-            t->w64[(size_t)P * ngp + Q] = w;
-            t->w32[(size_t)P * ngp + Q] = (float)w;
+            double w = m2[eri_index(pair_index(i, k), pair_index(j, l))] -
+                       m2[eri_index(pair_index(i, l), pair_index(j, k))];
+            if (i == k || i == l || j == k || j == l) {
+                if (j == l) w += h1(i, k);
+                if (i == k) w += h1(j, l);
+                if (j == k) w -= h1(i, l);
+                if (i == l) w -= h1(j, k);
+            } else {
+                t->w64[(size_t)P * ngp + Q] = w;
+                t->w32[(size_t)P * ngp + Q] = (float)w;
+            }
+            t->w64[nw + (size_t)P * ngp + Q] = w;
+            t->w32[nw + (size_t)P * ngp + Q] = (float)w;
         }
     JCI_CUDA(cudaMemcpyAsync(t->W64, t->w64.data(), t->w64.size() * sizeof(double),
                              cudaMemcpyHostToDevice, st));
@@ -500,27 +665,44 @@ int pair_block_cols(const PairTables &t, int len, int variant, size_t w) {
 }
 
 template <typename T>
-jci_status pair_launch(const PairTables &t, int len, int variant, const T *x, T *y, const T *hd,
-                       int add, const int *skip, T *E, int device, cudaStream_t st) {
+jci_status pair_launch(const PairTables &t, int len, int variant, int singles, const T *x, T *y,
+                       const T *hd, int add, const int *skip, T *E, int device, cudaStream_t st) {
     PairArgs<T> a;
     a.nk = t.nk; a.np = t.np; a.NP = t.NP; a.ngp = t.ngp; a.nt = t.nt;
     a.rows = t.rows; a.len = len;
     a.jrow = t.jrow; a.gp = t.gp; a.pull = t.pull;
     if constexpr (sizeof(T) == 8) a.W = t.W64;
     else a.W = t.W32;
+    if (singles) a.W += (size_t)t.ngp * t.ngp;
     a.skip = skip;
-    PairKernel<T> kern = pair_kernel<T>(t.NP / 16);
-    if (!kern) return JCI_ERR_SPACE;
-    const size_t smem = pair_smem<T>(t.NP);
-    int optin = 0;
+    const MmaKernel<T> mma = mma_kernel<T>(t.nf);
+    const PairKernel<T> wide = mma ? nullptr : pair_kernel<T>(t.NP / 16);
+    if (!mma && !wide) return JCI_ERR_SPACE;
+    const size_t smem = mma ? 2 * (size_t)((t.np + 3) / 4 * 4) * mma_ds<T>() * sizeof(T) +
+                                  (size_t)t.np * sizeof(int)
+                            : pair_smem<T>(t.NP);
+    int optin = 0, nsm = 0;
     JCI_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+    JCI_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
     if (smem > (size_t)optin) return JCI_ERR_SPACE;
-    JCI_CUDA(smem_optin(kern));
+    if (mma) JCI_CUDA(smem_optin(mma));
+    else JCI_CUDA(smem_optin(wide));
     const int cb = pair_block_cols(t, len, variant, sizeof(T));
     const size_t psmem = (size_t)kPullRows * t.nt * sizeof(int);
+    // 16-byte copies of X need rows that start and end on 16 bytes
+    const int vec = (size_t)len * sizeof(T) % 16 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0;
     for (int c0 = 0; c0 < len; c0 += cb) {
-        kern<<<t.nk, kPairThreads, smem, st>>>(a, x, E, c0, cb);
         const int w = std::min(cb, len - c0);
+        if (mma) {
+            // column segments until eight CTAs per SM, of at least four chunks
+            // (each builds its W_K, some 2 microseconds)
+            const int nch = (w + kPairCols - 1) / kPairCols;
+            const int ns = std::max(1, std::min(nch / 4, (8 * nsm + t.nk - 1) / t.nk));
+            const int seg = (nch + ns - 1) / ns * kPairCols;
+            mma<<<dim3(t.nk, (w + seg - 1) / seg), kMmaThreads, smem, st>>>(a, x, E, c0, cb, seg, vec);
+        } else {
+            wide<<<t.nk, kPairThreads, smem, st>>>(a, x, E, c0, cb);
+        }
         dim3 g((t.rows + kPullRows - 1) / kPullRows, (w + kPairThreads - 1) / kPairThreads);
         k_pairs_pull<T><<<g, kPairThreads, psmem, st>>>(a, E, x, y, hd, add, c0, cb);
     }
@@ -528,12 +710,130 @@ jci_status pair_launch(const PairTables &t, int len, int variant, const T *x, T 
     return JCI_OK;
 }
 
-template jci_status pair_launch<double>(const PairTables &, int, int, const double *, double *,
+template jci_status pair_launch<double>(const PairTables &, int, int, int, const double *, double *,
                                         const double *, int, const int *, double *, int,
                                         cudaStream_t);
-template jci_status pair_launch<float>(const PairTables &, int, int, const float *, float *,
+template jci_status pair_launch<float>(const PairTables &, int, int, int, const float *, float *,
                                        const float *, int, const int *, float *, int,
                                        cudaStream_t);
+
+// ---- singles' Coulomb part ---------------------------------------------------
+//
+// Y[r][i] (+)= sum_f s_f jc[pair_f][r] X[r][J_f] over the singles f of the
+// column string i (target J_f, phase s_f, pair_f): the part of hmatels_1x that
+// depends on the other spin's string r, sum_{m in r} (mm|pair); the part that
+// does not is in the hole-string products (pair_fill).  RB rows per CTA lie
+// interleaved in shared memory, so that one 16-byte load gives a target's
+// value in all of them and one load of a single's list entry serves them all;
+// lexically consecutive strings have mostly consecutive targets and the same
+// pair, so the loads meet few bank conflicts.  The row streams it replaces
+// read a whole row of X and one of jc from L2 for every single, at the L2's
+// bandwidth.  Measured, one spin's pass against the stream: FCI(14,14) FP64
+// 0.39 and 1.33 ms, FP32 0.27 and 0.81; FCI(16,16) FP64 6.4 and 25.1, FP32
+// 3.3 and 14.2; FCI(12,12) FP64 33 and 62 us.
+template <typename T>
+struct alignas(16) CoulVec {
+    T v[16 / sizeof(T)];
+};
+
+template <typename T>
+__global__ void __launch_bounds__(1024)
+    k_coulomb(int rows, int len, int ns, int npair, const uint32_t *__restrict__ list,
+              const T *__restrict__ jc, const T *__restrict__ X, T *__restrict__ Y, int add,
+              const int *skip) {
+    if (skip && *skip) return;
+    constexpr int RB = 16 / sizeof(T);
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T *xs = reinterpret_cast<T *>(smem_raw);      // [len][RB]
+    T *js = xs + (size_t)len * RB;                // [npair][RB]
+    const int r0 = blockIdx.x * RB, nt = blockDim.x, tid = threadIdx.x;
+    for (int r = 0; r < RB; r++) {
+        const bool in = r0 + r < rows;
+        const T *src = X + (long long)(r0 + r) * len;
+        for (int i = tid; i < len; i += nt) xs[(size_t)i * RB + r] = in ? src[i] : T(0);
+        for (int p = tid; p < npair; p += nt)
+            js[p * RB + r] = in ? jc[(long long)p * rows + r0 + r] : T(0);
+    }
+    __syncthreads();
+    const CoulVec<T> *xv = reinterpret_cast<const CoulVec<T> *>(xs);
+    const CoulVec<T> *jv = reinterpret_cast<const CoulVec<T> *>(js);
+    const int w = (len + gridDim.y - 1) / gridDim.y;
+    const int i1 = min(len, w * (int)(blockIdx.y + 1));
+    for (int i = w * blockIdx.y + tid; i < i1; i += nt) {
+        T acc[RB];
+#pragma unroll
+        for (int r = 0; r < RB; r++) acc[r] = T(0);
+        const uint32_t *pl = list + i;
+#pragma unroll 8
+        for (int f = 0; f < ns; f++) {
+            const uint32_t e = pl[(size_t)f * len];
+            const CoulVec<T> x = xv[e & 0xffffu], j = jv[(e >> 16) & 0x7fffu];
+#pragma unroll
+            for (int r = 0; r < RB; r++) {
+                if constexpr (sizeof(T) == 8)
+                    acc[r] = fma(__hiloint2double(__double2hiint(j.v[r]) ^ (int)(e & 0x80000000u),
+                                                  __double2loint(j.v[r])),
+                                 x.v[r], acc[r]);
+                else
+                    acc[r] = fmaf(__uint_as_float(__float_as_uint(j.v[r]) ^ (e & 0x80000000u)),
+                                  x.v[r], acc[r]);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < RB; r++)
+            if (r0 + r < rows) {
+                T *y = Y + (long long)(r0 + r) * len + i;
+                *y = add ? *y + acc[r] : acc[r];
+            }
+    }
+}
+
+// list[f][i] = target | pair << 16 | phase << 31
+__global__ void k_coulomb_list(long long n, const uint32_t *__restrict__ fs,
+                               const uint16_t *__restrict__ fp, uint32_t *list) {
+    const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (k < n)
+        list[k] = (fs[k] & 0x8000ffffu) | ((uint32_t)fp[k] << 16);
+}
+
+static size_t coulomb_smem_bytes(int len, int npair) { return (size_t)(len + npair) * 16; }
+
+bool coulomb_possible(int len, int npair, size_t smem_max) {
+    return len <= 65536 && npair < 32768 && coulomb_smem_bytes(len, npair) <= smem_max;
+}
+
+jci_status coulomb_list_build(int len, int ns, const uint32_t *fs, const uint16_t *fp,
+                              uint32_t **list, cudaStream_t st) {
+    const long long n = (long long)len * ns;
+    JCI_CUDA(cudaMalloc((void **)list, std::max<long long>(n, 1) * sizeof(uint32_t)));
+    if (n) k_coulomb_list<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, fs, fp, *list);
+    JCI_CUDA(cudaGetLastError());
+    return JCI_OK;
+}
+
+template <typename T>
+jci_status coulomb_launch(int rows, int len, int ns, int npair, const uint32_t *list, const T *jc,
+                          const T *x, T *y, int add, const int *skip, int device,
+                          cudaStream_t st) {
+    constexpr int RB = 16 / sizeof(T);
+    const size_t smem = coulomb_smem_bytes(len, npair);
+    JCI_CUDA(smem_optin(k_coulomb<T>));
+    int nsm = 0;
+    JCI_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
+    const int nt = len >= 4096 ? 1024 : len >= 512 ? 256 : 128;
+    const int gx = (rows + RB - 1) / RB;
+    // few rows: split the columns too (each CTA stages the rows again)
+    const int gy = std::max(1, std::min((len + nt - 1) / nt, 2 * nsm / gx));
+    k_coulomb<T><<<dim3(gx, gy), nt, smem, st>>>(rows, len, ns, npair, list, jc, x, y, add, skip);
+    JCI_CUDA(cudaGetLastError());
+    return JCI_OK;
+}
+template jci_status coulomb_launch<double>(int, int, int, int, const uint32_t *, const double *,
+                                           const double *, double *, int, const int *, int,
+                                           cudaStream_t);
+template jci_status coulomb_launch<float>(int, int, int, int, const uint32_t *, const float *,
+                                          const float *, float *, int, const int *, int,
+                                          cudaStream_t);
 
 // Single tables of one spin through its (N-1)-electron hole strings, in the
 // layout of the pair tables: hole strings in lexical order of the varying

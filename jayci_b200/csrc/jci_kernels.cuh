@@ -67,6 +67,35 @@ bool tc_possible(const AbShape &sh, int cw, size_t smem_max);
 jci_status tc_launch(const AbArgs<float> &a, int cw, int device, const float *v, float *o,
                      int *status, cudaStream_t st);
 
+// The fused product through 8-bit digits on the tcgen05 integer tensor cores
+// (jci_fci_i8.cu), FP64 and FP32.
+struct I8Tables {
+    int na = 0, nb = 0, npair = 0, nchunk = 0, nrow = 0, lmax = 0;
+    unsigned long long *mx = nullptr;       // largest integral of the panel, as bits
+    int *rowpair = nullptr;        // [128] pair of each panel row, -1: none
+    uint32_t *lofs = nullptr;      // [chunk + 1] first 16-byte unit of each chunk's lists
+    uint16_t *lists = nullptr;
+    uint8_t *eri[2] = {nullptr, nullptr};   // digits of the integrals, per precision
+    void *rscale[2] = {nullptr, nullptr};   // scale of the integrals
+    void *scratch[2] = {nullptr, nullptr};  // digits and scales of the vector
+};
+template <typename T>
+struct I8Input {
+    int sa;
+    const uint32_t *fsA;
+    const uint16_t *fpA;
+    const T *m2;
+    const int *skip;
+};
+jci_status i8_tables_build(const jci_space *s, int npair, I8Tables *t);
+void i8_tables_free(I8Tables *t);
+jci_status i8_fill(I8Tables *t, const double *m2, cudaStream_t st);
+size_t i8_smem(const I8Tables &t, int sa, size_t w);
+jci_status i8_scratch(I8Tables *t, size_t w);
+template <typename T>
+jci_status i8_launch(const I8Tables &t, const I8Input<T> &in, int device, const T *v, T *o,
+                     int *status, cudaStream_t st);
+
 // Same-spin doubles over groups of consecutive strings, jci_fci_group.cu.
 constexpr int kGroupRows = 16;
 template <typename T>
@@ -99,12 +128,12 @@ jci_status group_launch(const GroupArgs<T> &a, int items, int device, const T *x
 // Same-spin doubles through (N-2)-electron hole strings, jci_fci_pairs.cu
 // (group kernel variants 5 and 6).
 struct PairTables {
-    int nk = 0, np = 0, NP = 0, nt = 0, ngp = 0, rows = 0;
-    std::vector<int> orb;          // the varying orbitals (1-based)
+    int nk = 0, np = 0, NP = 0, nt = 0, ngp = 0, rows = 0, nf = 0, nv = 0;
+    std::vector<int> orb, fixed;   // the varying orbitals (1-based), those of every string
     int *jrow = nullptr;           // [hole string][pair] source string | phase << 31
     uint16_t *gp = nullptr;        // [hole string][pair] orbital pair
     int *pull = nullptr;           // [string][hole] hole string * np + pair
-    double *W64 = nullptr;         // [orbital pair][orbital pair]
+    double *W64 = nullptr;         // [doubles | with singles][orbital pair][orbital pair]
     float *W32 = nullptr;
     std::vector<double> w64;       // host copies behind the asynchronous uploads
     std::vector<float> w32;
@@ -115,8 +144,18 @@ void pair_tables_free(PairTables *t);
 size_t pair_smem_bytes(const PairTables &t, int prec);
 int pair_block_cols(const PairTables &t, int len, int variant, size_t w);
 template <typename T>
-jci_status pair_launch(const PairTables &t, int len, int variant, const T *x, T *y, const T *hd,
-                       int add, const int *skip, T *E, int device, cudaStream_t st);
+jci_status pair_launch(const PairTables &t, int len, int variant, int singles, const T *x, T *y,
+                       const T *hd, int add, const int *skip, T *E, int device, cudaStream_t st);
+
+// The singles' Coulomb part with the other spin's string (jci_fci_pairs.cu):
+// Y[r][i] (+)= sum_f s_f jc[pair_f][r] X[r][target_f] over the singles of i.
+bool coulomb_possible(int len, int npair, size_t smem_max);
+jci_status coulomb_list_build(int len, int ns, const uint32_t *fs, const uint16_t *fp,
+                              uint32_t **list, cudaStream_t st);
+template <typename T>
+jci_status coulomb_launch(int rows, int len, int ns, int npair, const uint32_t *list, const T *jc,
+                          const T *x, T *y, int add, const int *skip, int device,
+                          cudaStream_t st);
 
 // Singles of one spin through (N-1)-electron hole strings, jci_fci_pairs.cu
 // (the beta-singles pass of plans 6 and 7 with threads = 0).
