@@ -172,6 +172,7 @@ void device_free(jci_space *s) {
                  d->hdf, d->io_v, d->io_s};
     for (void *q : p) cudaFree(q);
     fci_free(d);
+    embed_free(d);
     davidson_free(d);
     if (d->ev0) cudaEventDestroy(d->ev0);
     if (d->ev1) cudaEventDestroy(d->ev1);
@@ -294,7 +295,7 @@ jci_status device_set_integrals(jci_space *s) {
     jci_status r = fci_prepare(s);
     if (r != JCI_OK) return r;
     JCI_CUDA(cudaStreamSynchronize(st));
-    return JCI_OK;
+    return embed_set_integrals(s);
 }
 
 jci_status device_hdiag(jci_space *s, double *d_out) {
@@ -440,6 +441,8 @@ jci_status device_sigma(jci_space *s, int nvec, const void *vin, void *sout, lon
     jci_status r = JCI_OK;
     if (d->single_group && fci_supported(s)) {
         r = fci_sigma(s, nvec, vin, sout, ld, precision, st);
+    } else if (!d->single_group && embed_chosen(s, vin, sout, ld, precision, st)) {
+        r = embed_sigma(s, nvec, vin, sout, ld, precision, st);
     } else if (precision == JCI_FP32) {
         launch_generic<float>(d, s->ndets, d->hdf, d->m2f, d->t[0].a1f, d->t[1].a1f,
                               (const float *)vin, (float *)sout, ld, nvec, st);

@@ -82,6 +82,7 @@ struct DeviceState {
     size_t io_bytes = 0;
     struct FciTables *fci = nullptr;   // single-group fast path (jci_fci.cu)
     struct DavidsonBuffers *dav = nullptr;  // jci_davidson.cu
+    struct Embedding *emb = nullptr;   // truncated spaces through the full space (jci_embed.cu)
     // Device flag read by every sigma kernel at entry: when nonzero the
     // kernel returns at once.  Set while a Davidson iteration is captured
     // into a CUDA graph, so that iterations launched after the solve has

@@ -99,6 +99,7 @@ jci_status fci_arm_wait_expiry(jci_space *s) {
 
 jci_status fci_wait_status(jci_space *s) {
     const DeviceState *d = s->dev;
+    if (d && d->emb) return embed_wait_status(d);
     if (!d || !d->fci || !d->fci->tc_status) return JCI_OK;
     int flag = 0;
     JCI_CUDA(cudaMemcpy(&flag, d->fci->tc_status, sizeof(int), cudaMemcpyDeviceToHost));

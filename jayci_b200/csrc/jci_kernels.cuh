@@ -181,6 +181,15 @@ jci_status hs_launch(const HsTables &t, int len, int npair, const T *jc, const T
 jci_status device_sigma_generic(jci_space *s, int nvec, const void *vin, void *sout,
                                 long long ld, int precision, cudaStream_t st);
 
+// Truncated spaces through the full CI space (jci_embed.cu).
+bool embed_chosen(jci_space *s, const void *v, void *o, long long ld, int precision,
+                  cudaStream_t st);
+jci_status embed_sigma(jci_space *s, int nvec, const void *v, void *o, long long ld, int precision,
+                       cudaStream_t st);
+jci_status embed_set_integrals(jci_space *s);
+jci_status embed_wait_status(const DeviceState *d);
+void embed_free(DeviceState *d);
+
 // Davidson buffers (jci_davidson.cu).
 void davidson_free(DeviceState *d);
 
