@@ -767,7 +767,9 @@ static jci_status sigma_block(Ctx &c, int i0, int m, bool fp32) {
             int mm = std::min(b->cap32, m - k0);
             k_d2f<<<grid_for(c.n), 256, 0, c.st>>>(b->V + (i0 + k0) * c.ld, b->v32, c.n, c.ld,
                                                    c.ld, mm, nullptr);
+            JCI_CUDA(cudaEventRecord(e0, c.st));
             if ((r = device_sigma(c.s, mm, b->v32, b->s32, c.ld, JCI_FP32, c.st))) return r;
+            JCI_CUDA(cudaEventRecord(e1, c.st));
             float ms = 0.f;
             JCI_CUDA(cudaEventSynchronize(e1));
             JCI_CUDA(cudaEventElapsedTime(&ms, e0, e1));
@@ -777,9 +779,11 @@ static jci_status sigma_block(Ctx &c, int i0, int m, bool fp32) {
         }
         c.fp32_vecs += m;
     } else {
+        JCI_CUDA(cudaEventRecord(e0, c.st));
         if ((r = device_sigma(c.s, m, b->V + i0 * c.ld, b->C + i0 * c.ld, c.ld, JCI_FP64,
                               c.st)))
             return r;
+        JCI_CUDA(cudaEventRecord(e1, c.st));
         float ms = 0.f;
         JCI_CUDA(cudaEventSynchronize(e1));
         JCI_CUDA(cudaEventElapsedTime(&ms, e0, e1));
@@ -1433,14 +1437,19 @@ jci_status davidson(jci_space *s, const jci_davidson_opts *o, double *energies, 
     if ((r = fci_wait_status(s))) return r;
     double core = s->nucrep + s->frzcore;
     for (int k = 0; k < o->nroots; k++) energies[k] = w[k] + core;
-    std::vector<double> host;
-    if (civec || o->write_files) {
-        host.resize((size_t)std::max(o->krymin, o->nroots) * c.n);
-        for (int k = 0; k < std::max(o->krymin, o->nroots); k++)
-            JCI_CUDA(cudaMemcpyAsync(&host[(size_t)k * c.n], c.b->V + k * c.ld,
-                                     c.n * sizeof(double), cudaMemcpyDeviceToHost, c.st));
+    if (civec) {
+        // straight into the caller's array: the roots only, no host copy between
+        JCI_CUDA(cudaMemcpy2DAsync(civec, c.n * sizeof(double), c.b->V, c.ld * sizeof(double),
+                                   c.n * sizeof(double), o->nroots, cudaMemcpyDeviceToHost, c.st));
         JCI_CUDA(cudaStreamSynchronize(c.st));
-        if (civec) memcpy(civec, host.data(), sizeof(double) * o->nroots * c.n);
+    }
+    std::vector<double> host;
+    if (o->write_files) {
+        const int nv = std::max(o->krymin, o->nroots);
+        host.resize((size_t)nv * c.n);
+        JCI_CUDA(cudaMemcpy2DAsync(host.data(), c.n * sizeof(double), c.b->V, c.ld * sizeof(double),
+                                   c.n * sizeof(double), nv, cudaMemcpyDeviceToHost, c.st));
+        JCI_CUDA(cudaStreamSynchronize(c.st));
     }
     if (o->write_files) {
         // pdavidson.c:343-347

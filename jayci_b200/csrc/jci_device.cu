@@ -169,7 +169,7 @@ void device_free(jci_space *s) {
         for (void *q : p) cudaFree(q);
     }
     void *p[] = {d->pairidx, d->pqoff, d->pqg, d->m1, d->m2, d->m1f, d->m2f, d->hd,
-                 d->hdf, d->io_v, d->io_s};
+                 d->hdf, d->io_v, d->io_s, d->dense, d->densef, d->dys};
     for (void *q : p) cudaFree(q);
     fci_free(d);
     embed_free(d);
@@ -260,6 +260,8 @@ __global__ void k_convert(const double *__restrict__ in, T *out, long long n) {
     if (i < n) out[i] = (T)in[i];
 }
 
+static jci_status dense_fill(jci_space *s);
+
 jci_status device_set_integrals(jci_space *s) {
     DeviceState *d = s->dev;
     JCI_CUDA(cudaSetDevice(d->device));
@@ -293,6 +295,7 @@ jci_status device_set_integrals(jci_space *s) {
                                                                d->m2, d->hd, d->hdf);
     JCI_CUDA(cudaGetLastError());
     jci_status r = fci_prepare(s);
+    if (r == JCI_OK) r = dense_fill(s);
     if (r != JCI_OK) return r;
     JCI_CUDA(cudaStreamSynchronize(st));
     return embed_set_integrals(s);
@@ -331,14 +334,12 @@ __device__ __forceinline__ T coul_other(const int *o, int ne, int pr, const T *m
     return s;
 }
 
-template <typename T, int NV>
-__global__ void __launch_bounds__(128)
-    k_sigma_generic(SpaceView v, const T *__restrict__ hd, const T *__restrict__ m2,
-                         const T *__restrict__ a1a, const T *__restrict__ a1b,
-                         const T *__restrict__ V, T *__restrict__ S, long long ld, int nvec) {
-    const long long d = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (d >= v.ndets || (v.skip && *v.skip)) return;
-    const int lane = threadIdx.x & 31;
+// add(h, j) for every off-diagonal element (i, j) of row d that falls to this
+// lane; each j once.
+template <typename T, typename F>
+__device__ __forceinline__ void generic_row(const SpaceView &v, long long d, int lane,
+                                            const T *__restrict__ m2, const T *__restrict__ a1a,
+                                            const T *__restrict__ a1b, F add) {
     int k = 0;
     while (k + 1 < v.npq && v.pqoff[k + 1] <= d) k++;
     const int pg = v.pqg[2 * k], qg = v.pqg[2 * k + 1];
@@ -347,14 +348,6 @@ __global__ void __launch_bounds__(128)
     const int p = v.a.gstart[pg] + (int)(r / nq), q = v.b.gstart[qg] + (int)(r % nq);
     const int *oa = v.a.istr + (long long)p * v.a.nelec;
     const int *ob = v.b.istr + (long long)q * v.b.nelec;
-    T acc[NV];
-#pragma unroll
-    for (int c = 0; c < NV; c++) acc[c] = T(0);
-    auto add = [&](T h, long long j) {
-#pragma unroll
-        for (int c = 0; c < NV; c++)
-            if (c < nvec) acc[c] += h * V[c * ld + j];
-    };
     auto dbl = [&](uint2 x) {
         const int i0 = x.y & 0xff, f0 = (x.y >> 8) & 0xff, i1 = (x.y >> 16) & 0xff, f1 = x.y >> 24;
         const T h = m2[eri_index(pair_index(i0, f0), pair_index(i1, f1))] -
@@ -402,11 +395,118 @@ __global__ void __launch_bounds__(128)
         const long long j = view_det(v, p, y.x & 0x3fffffff);
         if (j >= 0) add(dbl(y), j);
     }
+}
+
+template <typename T, int NV>
+__global__ void __launch_bounds__(128)
+    k_sigma_generic(SpaceView v, const T *__restrict__ hd, const T *__restrict__ m2,
+                    const T *__restrict__ a1a, const T *__restrict__ a1b,
+                    const T *__restrict__ V, T *__restrict__ S, long long ld, int nvec) {
+    const long long d = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (d >= v.ndets || (v.skip && *v.skip)) return;
+    const int lane = threadIdx.x & 31;
+    T acc[NV];
+#pragma unroll
+    for (int c = 0; c < NV; c++) acc[c] = T(0);
+    generic_row<T>(v, d, lane, m2, a1a, a1b, [&](T h, long long j) {
+#pragma unroll
+        for (int c = 0; c < NV; c++)
+            if (c < nvec) acc[c] += h * V[c * ld + j];
+    });
 #pragma unroll
     for (int c = 0; c < NV; c++) {
         for (int o = 16; o; o >>= 1) acc[c] += __shfl_xor_sync(~0u, acc[c], o);
         if (lane == 0 && c < nvec) S[c * ld + d] = fma(hd[d], V[c * ld + d], acc[c]);
     }
+}
+
+// ---- the smallest spaces ----------------------------------------------------
+//
+// Up to kDenseMax determinants the Hamiltonian itself is a table of at most
+// 32 MB, built from the integrals like the other tables, and sigma is one
+// launch that reads each row once: a warp per row.  The plans of the larger
+// spaces are two dependent launches, each a chain of table loads, whatever the
+// size: CAS(6,6), 400 determinants, 20.6 -> 11.4 us a call (18 us of kernels to 4; the
+// rest is the host).  Zero elements are skipped, so
+// that an infinity or NaN in c reaches the determinants it is connected to.
+constexpr long long kDenseMax = 2048;
+
+__global__ void __launch_bounds__(128)
+    k_dense_fill(SpaceView v, const double *__restrict__ hd, const double *__restrict__ m2,
+                 const double *__restrict__ a1a, const double *__restrict__ a1b, double *H,
+                 float *Hf, int ldh) {
+    const long long d = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (d >= v.ndets) return;
+    const int lane = threadIdx.x & 31;
+    double *row = H + d * ldh;
+    float *rowf = Hf + d * ldh;
+    const auto set = [&](double h, long long j) {
+        row[j] = h;
+        rowf[j] = (float)h;
+    };
+    generic_row<double>(v, d, lane, m2, a1a, a1b, set);
+    if (lane == 0) set(hd[d], d);
+}
+
+template <typename T, int NV>
+__global__ void __launch_bounds__(128)
+    k_sigma_dense(int n, int ldh, const T *__restrict__ H, const T *__restrict__ V,
+                  T *__restrict__ S, long long ld, int nvec, const int *skip) {
+    const int d = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (d >= n || (skip && *skip)) return;
+    const T *row = H + (long long)d * ldh;
+    T acc[NV];
+#pragma unroll
+    for (int c = 0; c < NV; c++) acc[c] = T(0);
+#pragma unroll 4
+    for (int j = lane; j < n; j += 32) {
+        const T h = row[j];
+#pragma unroll
+        for (int c = 0; c < NV; c++) {
+            const T x = c < nvec ? V[c * ld + j] : T(0);
+            if (h != T(0)) acc[c] = fma(h, x, acc[c]);
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < NV; c++) {
+        for (int o = 16; o; o >>= 1) acc[c] += __shfl_xor_sync(~0u, acc[c], o);
+        if (lane == 0 && c < nvec) S[c * ld + d] = acc[c];
+    }
+}
+
+template <typename T>
+static void launch_dense(const DeviceState *dv, int n, const T *H, const T *V, T *S, long long ld,
+                         int nvec, cudaStream_t st) {
+    const unsigned grid = (unsigned)((n + 3) / 4);
+    for (int c0 = 0; c0 < nvec; c0 += 4) {
+        const int nv = std::min(4, nvec - c0);
+        if (nv == 1)
+            k_sigma_dense<T, 1><<<grid, 128, 0, st>>>(n, dv->dense_ld, H, V + c0 * ld, S + c0 * ld,
+                                                     ld, nv, dv->sigma_skip);
+        else
+            k_sigma_dense<T, 4><<<grid, 128, 0, st>>>(n, dv->dense_ld, H, V + c0 * ld, S + c0 * ld,
+                                                     ld, nv, dv->sigma_skip);
+    }
+}
+
+static jci_status dense_fill(jci_space *s) {
+    DeviceState *d = s->dev;
+    if (s->ndets > kDenseMax) return JCI_OK;
+    cudaStream_t st = d->stream;
+    d->dense_ld = ((int)s->ndets + 31) / 32 * 32;
+    const size_t n = (size_t)s->ndets * d->dense_ld;
+    if (!d->dense) {
+        JCI_CUDA(cudaMalloc(&d->densef, n * sizeof(float)));
+        JCI_CUDA(cudaMalloc(&d->dense, n * sizeof(double)));
+    }
+    JCI_CUDA(cudaMemsetAsync(d->dense, 0, n * sizeof(double), st));
+    JCI_CUDA(cudaMemsetAsync(d->densef, 0, n * sizeof(float), st));
+    SpaceView v = make_view(d);
+    v.ndets = s->ndets;
+    k_dense_fill<<<(unsigned)((s->ndets + 3) / 4), 128, 0, st>>>(
+        v, d->hd, d->m2, d->t[0].a1, d->t[1].a1, d->dense, d->densef, d->dense_ld);
+    JCI_CUDA(cudaGetLastError());
+    return JCI_OK;
 }
 
 template <typename T>
@@ -433,13 +533,15 @@ jci_status device_sigma(jci_space *s, int nvec, const void *vin, void *sout, lon
     if (!s->have_ints) return JCI_ERR_STATE;
     if (nvec < 1 || ld < s->ndets || !vin || !sout) return JCI_ERR_ARG;
     cudaStream_t st = stream ? (cudaStream_t)stream : d->stream;
-    // no timing events while the stream is being captured into a graph
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    JCI_CUDA(cudaStreamIsCapturing(st, &cap));
-    const bool timed = cap == cudaStreamCaptureStatusNone;
-    if (timed) JCI_CUDA(cudaEventRecord(d->ev0, st));
     jci_status r = JCI_OK;
-    if (d->single_group && fci_supported(s)) {
+    if (d->dense && !fci_forced(s, precision)) {
+        if (precision == JCI_FP32)
+            launch_dense<float>(d, (int)s->ndets, d->densef, (const float *)vin, (float *)sout, ld,
+                                nvec, st);
+        else
+            launch_dense<double>(d, (int)s->ndets, d->dense, (const double *)vin, (double *)sout, ld,
+                                 nvec, st);
+    } else if (d->single_group && fci_supported(s)) {
         r = fci_sigma(s, nvec, vin, sout, ld, precision, st);
     } else if (!d->single_group && embed_chosen(s, vin, sout, ld, precision, st)) {
         r = embed_sigma(s, nvec, vin, sout, ld, precision, st);
@@ -452,7 +554,6 @@ jci_status device_sigma(jci_space *s, int nvec, const void *vin, void *sout, lon
     }
     if (r != JCI_OK) return r;
     JCI_CUDA(cudaGetLastError());
-    if (timed) JCI_CUDA(cudaEventRecord(d->ev1, st));
     return JCI_OK;
 }
 
@@ -468,14 +569,6 @@ jci_status device_sigma_generic(jci_space *s, int nvec, const void *vin, void *s
                                (const double *)vin, (double *)sout, ld, nvec, st);
     JCI_CUDA(cudaGetLastError());
     return JCI_OK;
-}
-
-float device_last_sigma_ms(jci_space *s) {
-    DeviceState *d = s->dev;
-    float ms = 0.f;
-    cudaEventSynchronize(d->ev1);
-    cudaEventElapsedTime(&ms, d->ev0, d->ev1);
-    return ms;
 }
 
 }  // namespace jci

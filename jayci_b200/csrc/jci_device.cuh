@@ -63,9 +63,8 @@ struct SpinTables {
 struct DeviceState {
     int device = 0;
     cudaStream_t stream = nullptr;
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr;  // the Davidson's sigma times
     cudaEvent_t evin = nullptr, evout = nullptr;  // ordering with the legacy default stream
-    float last_sigma_ms = 0.f;
     SpinTables t[2];
     int npq = 0;
     int *pairidx = nullptr;        // pegrps x qegrps
@@ -80,6 +79,11 @@ struct DeviceState {
     int *pqg = nullptr;            // npq x 2 group pair of each block
     void *io_v = nullptr, *io_s = nullptr;  // host-API staging buffers
     size_t io_bytes = 0;
+    void *dys = nullptr;           // jci_dyson's vectors and sums (grown on demand)
+    size_t dys_bytes = 0;
+    double *dense = nullptr;       // H itself, rows of dense_ld, for the smallest spaces
+    float *densef = nullptr;
+    int dense_ld = 0;
     struct FciTables *fci = nullptr;   // single-group fast path (jci_fci.cu)
     struct DavidsonBuffers *dav = nullptr;  // jci_davidson.cu
     struct Embedding *emb = nullptr;   // truncated spaces through the full space (jci_embed.cu)

@@ -48,6 +48,7 @@ struct FciTables {
     FciSpin<float> f[2];
     size_t smem_max = 0;
     bool tuned[2] = {false, false};                 // per precision (autotuned)
+    bool forced[2] = {false, false};                // fixed by the caller
     int tuned_nt[2] = {0, 0}, tuned_R[2] = {0, 0};
     int tuned_mode[2] = {0, 0}, tuned_B[2] = {1, 1};
     float tuned_ms[2] = {0.f, 0.f};
@@ -2613,6 +2614,11 @@ jci_status fci_sigma(jci_space *s, int nvec, const void *v, void *sig, long long
 // threads per CTA of the row kernel (modes 3, 4: of the alpha pass, B =
 // threads of the beta pass; modes 6, 7: of the beta-singles stream); R as
 // the product kernel takes it.
+bool fci_forced(const jci_space *s, int precision) {
+    const FciTables *f = s->dev ? s->dev->fci : nullptr;
+    return f && f->forced[precision == JCI_FP32 ? 1 : 0];
+}
+
 jci_status fci_force_plan(jci_space *s, int precision, int mode, int nt, int R, int B) {
     FciTables *f = s->dev ? s->dev->fci : nullptr;
     if (!f) return JCI_ERR_STATE;
@@ -2668,7 +2674,7 @@ jci_status fci_force_plan(jci_space *s, int precision, int mode, int nt, int R, 
         jci_status r = ab_tables(s, kMixBlock / 4, s->dev->stream, &t);
         if (r) return r;
     }
-    f->tuned[p] = true;
+    f->tuned[p] = f->forced[p] = true;
     f->tuned_mode[p] = mode;
     f->tuned_nt[p] = nt;
     f->tuned_R[p] = R;

@@ -73,7 +73,6 @@ void device_free(jci_space *s);
 jci_status device_hdiag(jci_space *s, double *d_out);  // device pointer
 jci_status device_sigma(jci_space *s, int nvec, const void *v, void *sig,
                         long long ld, int precision, void *stream);
-float device_last_sigma_ms(jci_space *s);
 jci_status davidson(jci_space *s, const jci_davidson_opts *o,
                     double *energies, double *civec, jci_davidson_stats *st);
 jci_status davidson_vectors(jci_space *s, int k, double *out);

@@ -23,6 +23,8 @@ jci_status fci_sigma(jci_space *s, int nvec, const void *v, void *sig, long long
 void fci_free(DeviceState *d);
 void fci_tuning(const jci_space *s, int precision, int *mode, int *nt, int *R, int *B,
                 float *ms);
+// Whether the caller fixed the plan of this precision (jci_sigma_set_plan).
+bool fci_forced(const jci_space *s, int precision);
 jci_status fci_force_plan(jci_space *s, int precision, int mode, int nt, int R, int B);
 jci_status fci_sigma_noalloc(jci_space *s, const void *v, void *o, int precision,
                              cudaStream_t st);
