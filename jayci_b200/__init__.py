@@ -213,13 +213,13 @@ class Space:
                                        nucrep, frzcore), "set_integrals")
 
     def hdiag(self):
-        out = np.zeros(self.ndets)
+        out = np.empty(self.ndets)
         _check(lib().jci_hdiag(self.h, _p(out)), "hdiag")
         return out
 
     def sigma(self, v, precision=FP64):
         v = np.ascontiguousarray(np.atleast_2d(v), np.float64)
-        out = np.zeros_like(v)
+        out = np.empty_like(v)
         _check(lib().jci_sigma(self.h, v.shape[0], _p(v), _p(out), precision), "sigma")
         return out
 
@@ -259,7 +259,7 @@ class Space:
             init = np.ascontiguousarray(init, np.float64)
             o.init = init.ctypes.data
         e = np.zeros(nroots)
-        civ = np.zeros((nroots, self.ndets)) if want_vectors else None
+        civ = np.empty((nroots, self.ndets)) if want_vectors else None
         st = DavidsonStats()
         r = lib().jci_davidson(self.h, ctypes.byref(o), _p(e),
                                _p(civ) if civ is not None else None, ctypes.byref(st))

@@ -103,15 +103,6 @@ __global__ void k_dyson_finish(const double *__restrict__ partial, int nblk, int
 
 using namespace jci;
 
-namespace {
-
-struct DevBuf {
-    void *p = nullptr;
-    ~DevBuf() { cudaFree(p); }
-};
-
-}  // namespace
-
 extern "C" jci_status jci_dyson(jci_space *s0, jci_space *s1, const double *v0, int nstates0,
                                 const double *v1, int nstates1, const int *states0, int nst0,
                                 const int *states1, int nst1, double *dyorb) {
@@ -156,33 +147,52 @@ extern "C" jci_status jci_dyson(jci_space *s0, jci_space *s1, const double *v0, 
     long long chunk = (n0 + kDysBlocks - 1) / kDysBlocks;
     chunk = (chunk + kDysThreads - 1) / kDysThreads * kDysThreads;
     const int nblk = (int)((n0 + chunk - 1) / chunk);
-    DevBuf dv0, dv1, drem, dpart, dout;
-    JCI_CUDA(cudaMalloc(&dv0.p, sizeof(double) * n0 * nst0));
-    JCI_CUDA(cudaMalloc(&dv1.p, sizeof(double) * n1 * nst1));
-    JCI_CUDA(cudaMalloc(&drem.p, sizeof(int) * rem.size()));
-    JCI_CUDA(cudaMalloc(&dpart.p, sizeof(double) * (size_t)nblk * norb * npr));
     const int norbs = s0->orbitals;
-    JCI_CUDA(cudaMalloc(&dout.p, sizeof(double) * (size_t)npr * norbs));
-    for (int j = 0; j < nst0; j++)
-        JCI_CUDA(cudaMemcpyAsync((double *)dv0.p + j * n0, v0 + (size_t)(states0[j] - 1) * n0,
-                                 sizeof(double) * n0, cudaMemcpyHostToDevice, stm));
-    for (int k = 0; k < nst1; k++)
-        JCI_CUDA(cudaMemcpyAsync((double *)dv1.p + k * n1, v1 + (size_t)(states1[k] - 1) * n1,
-                                 sizeof(double) * n1, cudaMemcpyHostToDevice, stm));
-    JCI_CUDA(cudaMemcpyAsync(drem.p, rem.data(), sizeof(int) * rem.size(),
-                             cudaMemcpyHostToDevice, stm));
-    JCI_CUDA(cudaMemsetAsync(dout.p, 0, sizeof(double) * (size_t)npr * norbs, stm));
+    // one buffer that stays with the handle: both vectors' states, the removal
+    // table, the partial sums, the result (256-byte aligned parts)
+    const size_t sizes[5] = {sizeof(double) * n0 * nst0, sizeof(double) * n1 * nst1,
+                             sizeof(int) * rem.size(), sizeof(double) * (size_t)nblk * norb * npr,
+                             sizeof(double) * (size_t)npr * norbs};
+    size_t offs[6] = {0};
+    for (int i = 0; i < 5; i++) offs[i + 1] = offs[i] + (sizes[i] + 255) / 256 * 256;
+    if (d0->dys_bytes < offs[5]) {
+        cudaFree(d0->dys);
+        d0->dys = nullptr;
+        d0->dys_bytes = 0;
+        JCI_CUDA(cudaMalloc(&d0->dys, offs[5]));
+        d0->dys_bytes = offs[5];
+    }
+    char *base = (char *)d0->dys;
+    double *dv0 = (double *)base, *dv1 = (double *)(base + offs[1]);
+    int *drem = (int *)(base + offs[2]);
+    double *dpart = (double *)(base + offs[3]), *dout = (double *)(base + offs[4]);
+    // consecutive states travel in one copy
+    auto upload = [&](double *dst, const double *src, const int *states, int nst, long long n) {
+        for (int j = 0; j < nst;) {
+            int m = 1;
+            while (j + m < nst && states[j + m] == states[j] + m) m++;
+            const cudaError_t e =
+                cudaMemcpyAsync(dst + j * n, src + (size_t)(states[j] - 1) * n,
+                                sizeof(double) * n * m, cudaMemcpyHostToDevice, stm);
+            if (e != cudaSuccess) return e;
+            j += m;
+        }
+        return cudaSuccess;
+    };
+    JCI_CUDA(upload(dv0, v0, states0, nst0, n0));
+    JCI_CUDA(upload(dv1, v1, states1, nst1, n1));
+    JCI_CUDA(cudaMemcpyAsync(drem, rem.data(), sizeof(int) * rem.size(), cudaMemcpyHostToDevice,
+                             stm));
+    JCI_CUDA(cudaMemsetAsync(dout, 0, sizes[4], stm));
     SpaceView w0 = make_view(s0->dev), w1 = make_view(s1->dev);
     w0.ndets = n0;
     w1.ndets = n1;
-    k_dyson<<<nblk, kDysThreads, 0, stm>>>(w0, w1, sp, (const int *)drem.p, norb,
-                                           (const double *)dv0.p, nst0, (const double *)dv1.p,
-                                           nst1, chunk, (double *)dpart.p);
-    k_dyson_finish<<<norb * npr, 32, 0, stm>>>((const double *)dpart.p, nblk, norb, npr, norbs,
-                                               sqrt((double)s0->electrons), (double *)dout.p);
+    k_dyson<<<nblk, kDysThreads, 0, stm>>>(w0, w1, sp, drem, norb, dv0, nst0, dv1, nst1, chunk,
+                                           dpart);
+    k_dyson_finish<<<norb * npr, 32, 0, stm>>>(dpart, nblk, norb, npr, norbs,
+                                               sqrt((double)s0->electrons), dout);
     JCI_CUDA(cudaGetLastError());
-    JCI_CUDA(cudaMemcpyAsync(dyorb, dout.p, sizeof(double) * (size_t)npr * norbs,
-                             cudaMemcpyDeviceToHost, stm));
+    JCI_CUDA(cudaMemcpyAsync(dyorb, dout, sizes[4], cudaMemcpyDeviceToHost, stm));
     JCI_CUDA(cudaStreamSynchronize(stm));
     return JCI_OK;
 }
