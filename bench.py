@@ -79,6 +79,8 @@ def sigma_plan_desc(mode, nt, R, B, ms=None):
     d = {"mode": mode, "name": PLAN_NAMES[mode],
          ("alpha_pass_threads" if streams else "beta_singles_threads" if groups
           else "row_kernel_threads"): nt}
+    if mode == 5 and nt == 1:
+        d["same_spin"] = "dense products of the string matrices"
     if groups and nt == 1:
         d["singles"] = "same-spin part in the hole-string products, Coulomb pass"
     elif groups and nt == 0:

@@ -208,7 +208,9 @@ jci_status jci_sigma_device_noalloc(jci_space *s, const void *v, void *sigma,
  * 3-4: of the alpha pass; modes 6-7: of the beta-singles stream, or 0 for
  * the beta singles as products over (N-1)-electron hole strings, or, mode 7
  * with rows 128 and batch 5-7, 1 for the singles of both spins split between
- * the hole-string products and a Coulomb pass), `rows`
+ * the hole-string products and a Coulomb pass; mode 5 with batch 1, 1 for the
+ * same-spin part as dense products over at most 2048 strings of a spin in
+ * place of the row kernel), `rows`
  * (mode 0: alpha rows staged per pass; modes 1-3 and 6: product CTAs per
  * SM, 0 = as many as fit, plus 16 for the panel cut into 256-column blocks
  * gathered block by block, plus 32 for one panel per alpha row built and
@@ -228,8 +230,9 @@ jci_status jci_sigma_device_noalloc(jci_space *s, const void *v, void *sigma,
  * strings, in the widest column blocks whose scratch fits 1 GiB (5) or
  * 4 GiB (7), or in 64-column blocks (6)), and
  * its timed cost in
- * ms per vector.  All 0 before the first sigma call and on the
- * multi-group path.  No reference counterpart (the reference has no device
+ * ms per vector.  All 0 before the first sigma call, on the
+ * multi-group path and for spaces of at most 2048 determinants (one dense
+ * product) unless a plan is set.  No reference counterpart (the reference has no device
  * tuning). */
 jci_status jci_sigma_tuning(const jci_space *s, int precision, int *mode,
                             int *threads, int *rows, int *batch, float *ms);

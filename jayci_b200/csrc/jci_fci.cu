@@ -84,6 +84,8 @@ struct FciTables {
     I8Tables i8;                   // fused product on the integer tensor cores
     int i8_state = 0;              // as prs_state
     uint32_t *clist[2] = {nullptr, nullptr};  // singles of each spin for k_coulomb
+    SameDense sd;                  // same-spin matrices of short string lists
+    int sd_state = 0;              // as prs_state
 };
 
 bool fci_supported(const jci_space *s) {
@@ -145,6 +147,7 @@ void fci_free(DeviceState *d) {
     i8_tables_free(&f->i8);
     cudaFree(f->clist[0]);
     cudaFree(f->clist[1]);
+    same_dense_free(&f->sd);
     delete f;
     d->fci = nullptr;
 }
@@ -1442,6 +1445,11 @@ jci_status fci_prepare(jci_space *s) {
             jci_status r = pair_fill(s, &f->prs[sp], st);
             if (r) return r;
         }
+        if (f->sd_state == 1) {
+            jci_status r = same_dense_fill(&f->sd, sp, X.max_sing, X.max_doub, t.fsing, f->d[sp].a1T,
+                                           f->dblJ[sp], f->d[sp].dblH, st);
+            if (r) return r;
+        }
         if (sp == 1 && f->i8_state == 1) {
             jci_status r = i8_fill(&f->i8, d->m2, st);
             if (r) return r;
@@ -2214,6 +2222,39 @@ static jci_status launch_coulomb(jci_space *s, const FciArgs<T> &a, int sp, int 
                              s->dev->device, st);
 }
 
+// The same-spin matrices of both spins, built and filled on first use (not
+// while a stream is being captured); JCI_ERR_SPACE, and remembered, for longer
+// string lists.
+static jci_status same_dense(jci_space *s, cudaStream_t st) {
+    FciTables *f = s->dev->fci;
+    if (f->sd_state) return f->sd_state > 0 ? JCI_OK : JCI_ERR_SPACE;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    JCI_CUDA(cudaStreamIsCapturing(st, &cs));
+    if (cs != cudaStreamCaptureStatusNone) return JCI_ERR_STATE;
+    if (f->na > kSameDenseMax || f->nb > kSameDenseMax) {
+        f->sd_state = -1;
+        return JCI_ERR_SPACE;
+    }
+    jci_status r = JCI_OK;
+    for (int sp = 0; sp < 2 && !r; sp++) {
+        r = same_dense_build(&f->sd, sp, sp == 0 ? f->na : f->nb);
+        if (!r)
+            r = same_dense_fill(&f->sd, sp, sp == 0 ? f->sa : f->sb, sp == 0 ? f->da : f->db,
+                                s->dev->t[sp].fsing, f->d[sp].a1T, f->dblJ[sp], f->d[sp].dblH, st);
+    }
+    const size_t zn = ((size_t)f->sa * f->na + 1) * sizeof(double);
+    if (!r && (cudaMalloc(&f->sd.zero, zn) != cudaSuccess ||
+               cudaMemsetAsync(f->sd.zero, 0, zn, st) != cudaSuccess))
+        r = JCI_ERR_NOMEM;
+    if (r) {
+        cudaGetLastError();
+        same_dense_free(&f->sd);
+        return r;
+    }
+    f->sd_state = 1;
+    return JCI_OK;
+}
+
 // One full sigma of one vector with the given plan.
 // mode 0: k_sigma_fci with R staged alpha rows.
 // modes 1, 2, 5: k_sigma_rows (nt threads, B rows per CTA), then the product:
@@ -2228,7 +2269,9 @@ static jci_status launch_coulomb(jci_space *s, const FciArgs<T> &a, int sp, int 
 //   stream on C^T (nt threads), then the product of mode 3 (6) or of
 //   mode 4 (7).  Mode 7 with nt = 1 (integer engine, hole-string doubles):
 //   the singles of both spins split between the hole-string products and
-//   k_coulomb.
+//   k_coulomb.  Mode 5 with nt = 1: the same-spin part as dense products
+//   (jci_fci_dense.cu) instead of the row kernel, the singles' Coulomb part by
+//   k_coulomb (the alpha ones' by the product where its engine has them).
 template <typename T>
 static jci_status run_plan(jci_space *s, FciArgs<T> a, int mode, int nt, int R, int B,
                            const T *v, T *o, cudaStream_t st) {
@@ -2283,6 +2326,21 @@ static jci_status run_plan(jci_space *s, FciArgs<T> a, int mode, int nt, int R, 
     }
     a.do_as = 0;
     a.R = 0;
+    if (nt == kSplitSingles) {  // mode 5
+        if ((r = same_dense(s, st))) return r;
+        if ((r = launch_coulomb<T>(s, a, 1, 0, v, o, st))) return r;
+        a.a1A = (const T *)f->sd.zero;  // in the same-spin product
+        if ((r = launch_ab<T>(s, a, v, o, st, R, false))) return r;
+        if (R == kI8Engine) {  // leaves out the alpha singles' Coulomb part
+            T *ct, *tau;
+            if ((r = stream_scratch<T>(f, &ct, &tau))) return r;
+            if ((r = launch_transposes<T>(f, v, ct, o, tau, false, a.skip, st))) return r;
+            if ((r = launch_coulomb<T>(s, a, 0, 0, ct, tau, st))) return r;
+            if ((r = launch_transposes<T>(f, v, ct, o, tau, true, a.skip, st))) return r;
+        }
+        // the diagonal, the largest term, last
+        return same_dense_launch<T>(f->sd, a.hd, a.skip, s->dev->device, v, o, st);
+    }
     if ((r = launch_rows<T>(a, nt, B, v, o, st))) return r;
     if (mode == 2) return launch_mixed2<T>(s, a, v, o, st, R);
     if (mode == 5) return launch_ab<T>(s, a, v, o, st, R);
@@ -2487,6 +2545,21 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
         if (found && gg < 1e30f) best6 = bs + gg + tt + bsprod;
         err = JCI_OK;  // a space the group tables cannot hold just drops the plan
     }
+    // mode 5 with the same-spin part as dense products, end to end.  Measured
+    // (us, best of the other plans -> this one): N electrons in N orbitals
+    // FP64 N = 8 32 -> 28, 9 38 -> 29, 10 64 -> 47, 11 163 -> 145, 12 549 -> 488;
+    // FP32 9 37 -> 30, 10 57 -> 42, 11 142 -> 131, 12 398 -> 385; 8 in 13
+    // orbitals FP64 379 -> 336.  At N = 13 (1 716 strings) the lists win.
+    float bestd = 1e30f;
+    int bdR = 0;
+    if (!only_split && coulomb_lists(s, st) == JCI_OK && same_dense(s, st) == JCI_OK) {
+        for (int tx : {8, 16, 32, 64, kI8Engine}) {
+            if (!ab_plan_possible(s, tx, w, st)) continue;
+            const float ms =
+                best_of([&] { return run_plan<T>(s, a, 5, kSplitSingles, tx, 1, v, o, st); });
+            if (ms < bestd) { bestd = ms; bdR = tx; }
+        }
+    }
     const int gmode = sab ? 7 : 6;
     if (b0nt) best0 = best_of([&] { return run_plan<T>(s, a, 0, b0nt, b0R, 1, v, o, st); });
     if (b1nt)
@@ -2508,7 +2581,8 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
     cudaFree(v);
     cudaFree(o);
     if (err) return err;
-    if (!b0nt && !b1nt && !(b3a && b3b) && best6 >= 1e30f && bests >= 1e30f)
+    if (!b0nt && !b1nt && !(b3a && b3b) && best6 >= 1e30f && bests >= 1e30f &&
+        bestd >= 1e30f)
         return JCI_ERR_SPACE;
     int mode = 0;
     float best = best0;
@@ -2522,11 +2596,19 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
         b6s = kSplitSingles;
         b6i = bsB;
     }
+    const bool dense = bestd < best;
+    if (dense) {
+        mode = 5;
+        best = bestd;
+        b1nt = kSplitSingles;
+        b1R = bdR;
+        b1B = 1;
+    }
     const bool streams = mode == 3 || mode == 4, groups = mode == 6 || mode == 7;
     f->tuned[prec] = true;
     f->tuned_mode[prec] = mode;
     f->tuned_nt[prec] = groups ? b6s : streams ? b3a : mode ? b1nt : b0nt;
-    f->tuned_R[prec] = split ? kI8Engine : (streams || groups) ? sR : mode ? b1R : b0R;
+    f->tuned_R[prec] = split && groups ? kI8Engine : (streams || groups) ? sR : mode ? b1R : b0R;
     f->tuned_B[prec] = groups ? b6i : streams ? b3b : mode ? b1B : 1;
     f->tuned_ms[prec] = best;
     // drop the group tables unless a precision uses them
@@ -2534,6 +2616,12 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
     if (!groups && other != 6 && other != 7) {
         group_tables_free(&f->grp[0]);
         group_tables_free(&f->grp[1]);
+    }
+    // nor the same-spin matrices
+    if (!dense && f->sd_state == 1 &&
+        !(f->tuned_mode[prec ^ 1] == 5 && f->tuned_nt[prec ^ 1] == kSplitSingles)) {
+        same_dense_free(&f->sd);
+        f->sd_state = 0;
     }
     const int eng = mode == 4 || mode == 5 || mode == 7 ? f->tuned_R[prec] : 0;
     if (eng != kI8Engine && f->i8.scratch[prec]) {  // the integer engine's digits are not needed
@@ -2545,7 +2633,7 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
         f->tbuf[prec] = nullptr;
         f->mix_grid[prec] = 0;
     }
-    if (!streams && !groups && f->sbuf[prec]) {  // the streaming scratch is not needed
+    if (!streams && !groups && !(dense && bdR == kI8Engine) && f->sbuf[prec]) {  // the streaming scratch is not needed
         cudaFree(f->sbuf[prec]);
         f->sbuf[prec] = nullptr;
     }
@@ -2644,7 +2732,11 @@ jci_status fci_force_plan(jci_space *s, int precision, int mode, int nt, int R, 
         bool ok = mode == 1   ? mixed_possible(f, w) && R >= 0
                   : mode == 2 ? mixed2_possible(f, w) && R >= 0
                               : ab_plan_possible(s, R, w, s->dev->stream);
-        if (!ok || !rows_ok(f->nb, nt, B) || rows_smem(f->nb, f->npair, f->da, B, w) > f->smem_max)
+        if (mode == 5 && nt == kSplitSingles) {
+            if (!ok || B != 1 || coulomb_lists(s, s->dev->stream) != JCI_OK ||
+                same_dense(s, s->dev->stream) != JCI_OK)
+                return JCI_ERR_ARG;
+        } else if (!ok || !rows_ok(f->nb, nt, B) || rows_smem(f->nb, f->npair, f->da, B, w) > f->smem_max)
             return JCI_ERR_ARG;
     } else {
         int items = (f->nb + nt - 1) / nt;

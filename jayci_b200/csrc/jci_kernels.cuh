@@ -183,6 +183,23 @@ jci_status hs_launch(const HsTables &t, int len, int npair, const T *jc, const T
 jci_status device_sigma_generic(jci_space *s, int nvec, const void *vin, void *sout,
                                 long long ld, int precision, cudaStream_t st);
 
+// The same-spin part of the one-group sigma as dense products (jci_fci_dense.cu).
+constexpr int kSameDenseMax = 2048;  // strings of a spin, at most
+struct SameDense {
+    int n[2] = {0, 0}, ld[2] = {0, 0};
+    double *H64[2] = {nullptr, nullptr};   // [string][ld] singles and doubles of the spin
+    float *H32[2] = {nullptr, nullptr};
+    void *zero = nullptr;                  // [single][string] zeros: no one-body part elsewhere
+};
+jci_status same_dense_build(SameDense *t, int spin, int nstr);
+void same_dense_free(SameDense *t);
+jci_status same_dense_fill(SameDense *t, int spin, int ns, int nd, const uint32_t *fs,
+                           const double *a1T, const int *dblJ, const double *dblH,
+                           cudaStream_t st);
+template <typename T>
+jci_status same_dense_launch(const SameDense &t, const T *hd, const int *skip, int device,
+                             const T *x, T *y, cudaStream_t st);
+
 // Truncated spaces through the full CI space (jci_embed.cu).
 bool embed_chosen(jci_space *s, const void *v, void *o, long long ld, int precision,
                   cudaStream_t st);
