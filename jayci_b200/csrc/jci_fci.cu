@@ -1952,7 +1952,8 @@ static jci_status ab_tables(jci_space *s, int tx, cudaStream_t st, AbTables **ou
 // from a row stream here unless the plan takes them elsewhere (singles = 0).
 template <typename T>
 static jci_status launch_ab(jci_space *s, const FciArgs<T> &fa, const T *v, T *o,
-                            cudaStream_t st, int tx, bool singles = true) {
+                            cudaStream_t st, int tx, bool singles = true,
+                            const T *jself = nullptr) {
     AbTables *t = nullptr;
     const bool tc = is_tc_engine(tx);
     if (tx == kI8Engine) {
@@ -1981,6 +1982,7 @@ static jci_status launch_ab(jci_space *s, const FciArgs<T> &fa, const T *v, T *o
     m.fsA = fa.fsA; m.fpA = fa.fpA; m.a1A = fa.a1A; m.m2 = fa.m2;
     m.off = t->off; m.base = t->base; m.ent = t->ent;
     m.skip = fa.skip;
+    m.jself = jself;
     if constexpr (sizeof(T) == sizeof(float)) {
         if (tc) {
             return tc_launch(m, tx, s->dev->device, v, o, s->dev->fci->tc_status, st);
@@ -2271,7 +2273,7 @@ static jci_status same_dense(jci_space *s, cudaStream_t st) {
 //   the singles of both spins split between the hole-string products and
 //   k_coulomb.  Mode 5 with nt = 1: the same-spin part as dense products
 //   (jci_fci_dense.cu) instead of the row kernel, the singles' Coulomb part by
-//   k_coulomb (the alpha ones' by the product where its engine has them).
+//   k_coulomb or, where its engine and sizes allow (ab_self), by the product.
 template <typename T>
 static jci_status run_plan(jci_space *s, FciArgs<T> a, int mode, int nt, int R, int B,
                            const T *v, T *o, cudaStream_t st) {
@@ -2328,9 +2330,11 @@ static jci_status run_plan(jci_space *s, FciArgs<T> a, int mode, int nt, int R, 
     a.R = 0;
     if (nt == kSplitSingles) {  // mode 5
         if ((r = same_dense(s, st))) return r;
-        if ((r = launch_coulomb<T>(s, a, 1, 0, v, o, st))) return r;
+        const AbShape sh{f->nb, f->sa, f->sb, f->nelb, f->npair};
+        const bool self = ab_self(sh, s->ndets, R, w, f->smem_max);
+        if (!self && (r = launch_coulomb<T>(s, a, 1, 0, v, o, st))) return r;
         a.a1A = (const T *)f->sd.zero;  // in the same-spin product
-        if ((r = launch_ab<T>(s, a, v, o, st, R, false))) return r;
+        if ((r = launch_ab<T>(s, a, v, o, st, R, false, self ? a.jA : nullptr))) return r;
         if (R == kI8Engine) {  // leaves out the alpha singles' Coulomb part
             T *ct, *tau;
             if ((r = stream_scratch<T>(f, &ct, &tau))) return r;
@@ -2547,9 +2551,9 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
     }
     // mode 5 with the same-spin part as dense products, end to end.  Measured
     // (us, best of the other plans -> this one): N electrons in N orbitals
-    // FP64 N = 8 32 -> 28, 9 38 -> 29, 10 64 -> 47, 11 163 -> 145, 12 549 -> 488;
-    // FP32 9 37 -> 30, 10 57 -> 42, 11 142 -> 131, 12 398 -> 385; 8 in 13
-    // orbitals FP64 379 -> 336.  At N = 13 (1 716 strings) the lists win.
+    // FP64 N = 8 32 -> 24, 9 38 -> 24, 10 64 -> 40, 11 163 -> 130, 12 549 -> 488;
+    // FP32 9 37 -> 24, 10 57 -> 36, 11 142 -> 118, 12 398 -> 385; 8 in 13
+    // orbitals FP64 379 -> 335.  At N = 13 (1 716 strings) the lists win.
     float bestd = 1e30f;
     int bdR = 0;
     if (!only_split && coulomb_lists(s, st) == JCI_OK && same_dense(s, st) == JCI_OK) {

@@ -49,6 +49,21 @@ __device__ __forceinline__ void ab_dmma(double (&d)[2], double a, double b) {
                  : "d"(a), "d"(b));
 }
 
+// Columns of the product: the alpha singles and, with SELF (the tensor-core
+// engines; jself is then set), the string itself, whose entry in the row of pair p is
+// sum_{m in Ia} (mm|p): the gather then adds the beta singles' Coulomb part
+// (hmatels_1x), which k_coulomb would otherwise sum up in a pass of its own
+// (9 us of 47 at 63 504 determinants).  Its entries in the rows (mm) are zero:
+// what they would add is the diagonal's.
+__device__ __forceinline__ bool ab_diagonal_row(int m) {  // m = p (p + 1) / 2 - 1
+    const int p = (int)sqrtf(2.f * (m + 1));
+    return p * (p + 1) / 2 == m + 1;
+}
+template <typename T>
+__device__ __forceinline__ T ab_self_a(const AbArgs<T> &a, int Ia, int m) {
+    return m < a.npair && !ab_diagonal_row(m) ? a.jself[(long long)m * a.na + Ia] : T(0);
+}
+
 // ---- CUDA-core engine -------------------------------------------------------
 //
 // TX threads across the chunk's columns (4 consecutive columns each, so
@@ -199,13 +214,13 @@ __host__ __device__ inline int dm_kp(int K) {
     return k4 + (20 - k4 % 16) % 16;
 }
 
-template <int MTW, int ITEMS, int NB>
+template <int MTW, int ITEMS, int NB, bool SELF>
 __global__ void __launch_bounds__(kAbThreads, NB == 1 ? 2 : 1)  // one B buffer: two CTAs per SM
     k_sigma_ab_dmma(AbArgs<double> a, const double *__restrict__ V, double *__restrict__ S) {
     if (a.skip && *a.skip) return;
     constexpr int R8 = 16 * MTW;  // product rows covered (>= mrows)
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int K = a.sa, K4 = dm_k4(K), KP = dm_kp(K), nb = a.nb;
+    const int K = a.sa + SELF, K4 = dm_k4(K), KP = dm_kp(K), nb = a.nb;
     double *As = reinterpret_cast<double *>(smem_raw);             // [R8][KP]
     double *Bs = As + (size_t)R8 * KP;                             // [NB][K4][kDmCWP]
     double *Ts = Bs + NB * (size_t)K4 * kDmCWP;                    // [mrows][kDmCW]
@@ -258,15 +273,18 @@ __global__ void __launch_bounds__(kAbThreads, NB == 1 ? 2 : 1)  // one B buffer:
         for (int idx = tid; idx < R8 * K4; idx += kAbThreads) {
             const int m = idx / K4, j = idx - m * K4;
             double v = 0.0;
-            if (j < K && m <= a.npair) {
+            if (j < a.sa && m <= a.npair) {
                 const long long o = (long long)j * a.na + Ia;
                 v = m < a.npair ? a.m2[eri_index(a.fpA[o], m)] : a.a1A[o];
                 if (a.fsA[o] >> 31) v = -v;
+            } else if (SELF && j == a.sa) {
+                v = ab_self_a(a, Ia, m);
             }
             As[(size_t)m * KP + j] = v;
         }
         for (int j = tid; j < K; j += kAbThreads)
-            jl[j] = (int)(a.fsA[(long long)j * a.na + Ia] & 0x3fffffffu);
+            jl[j] = SELF && j == a.sa ? Ia
+                                       : (int)(a.fsA[(long long)j * a.na + Ia] & 0x3fffffffu);
         double x[ITEMS];
 #pragma unroll
         for (int i = 0; i < ITEMS; i++) x[i] = 0.0;
@@ -338,7 +356,7 @@ __global__ void __launch_bounds__(kAbThreads, NB == 1 ? 2 : 1)  // one B buffer:
 #pragma unroll
         for (int i = 0; i < ITEMS; i++) {
             const int Ib = tid + kAbThreads * i;
-            if (Ib < nb) srow[Ib] += x[i];
+            if (Ib < nb) srow[Ib] = SELF ? x[i] : srow[Ib] + x[i];
         }
     }
 }
@@ -384,13 +402,13 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], 
 
 // AS = 1: the A panel is split once per alpha string and kept as its TF32
 // parts (two panels); AS = 0: A is kept in FP32 and split at every load.
-template <int MT, int ITEMS, int NB, int AS>
+template <int MT, int ITEMS, int NB, int AS, bool SELF>
 __global__ void __launch_bounds__(kAbThreads, NB == 1 ? 2 : 1)  // one B buffer: two CTAs per SM
     k_sigma_ab_tf32(AbArgs<float> a, const float *__restrict__ V, float *__restrict__ S) {
     if (a.skip && *a.skip) return;
     constexpr int R16 = 32 * MT;  // product rows covered (>= mrows)
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int K = a.sa, K8 = tf_k8(K), KP = tf_kp(K), nb = a.nb;
+    const int K = a.sa + SELF, K8 = tf_k8(K), KP = tf_kp(K), nb = a.nb;
     float *As = reinterpret_cast<float *>(smem_raw);               // [1 + AS][R16][KP]
     uint32_t *Ah = reinterpret_cast<uint32_t *>(As);               // AS: TF32 high parts
     uint32_t *Al = Ah + (size_t)R16 * KP;                          // AS: TF32 remainders
@@ -443,10 +461,12 @@ __global__ void __launch_bounds__(kAbThreads, NB == 1 ? 2 : 1)  // one B buffer:
         for (int idx = tid; idx < R16 * K8; idx += kAbThreads) {
             const int m = idx / K8, j = idx - m * K8;
             float v = 0.f;
-            if (j < K && m <= a.npair) {
+            if (j < a.sa && m <= a.npair) {
                 const long long o = (long long)j * a.na + Ia;
                 v = m < a.npair ? a.m2[eri_index(a.fpA[o], m)] : a.a1A[o];
                 if (a.fsA[o] >> 31) v = -v;
+            } else if (SELF && j == a.sa) {
+                v = ab_self_a(a, Ia, m);
             }
             if (AS)
                 split_tf32(v, Ah[(size_t)m * KP + j], Al[(size_t)m * KP + j]);
@@ -454,7 +474,8 @@ __global__ void __launch_bounds__(kAbThreads, NB == 1 ? 2 : 1)  // one B buffer:
                 As[(size_t)m * KP + j] = v;
         }
         for (int j = tid; j < K; j += kAbThreads)
-            jl[j] = (int)(a.fsA[(long long)j * a.na + Ia] & 0x3fffffffu);
+            jl[j] = SELF && j == a.sa ? Ia
+                                       : (int)(a.fsA[(long long)j * a.na + Ia] & 0x3fffffffu);
         float x[ITEMS];
 #pragma unroll
         for (int i = 0; i < ITEMS; i++) x[i] = 0.f;
@@ -547,7 +568,7 @@ __global__ void __launch_bounds__(kAbThreads, NB == 1 ? 2 : 1)  // one B buffer:
 #pragma unroll
         for (int i = 0; i < ITEMS; i++) {
             const int Ib = tid + kAbThreads * i;
-            if (Ib < nb) srow[Ib] += x[i];
+            if (Ib < nb) srow[Ib] = SELF ? x[i] : srow[Ib] + x[i];
         }
     }
 }
@@ -577,30 +598,30 @@ AbKernel<T> ab_kernel_tm(int tm) {
     return nullptr;
 }
 
-template <int ITEMS, int NB>
+template <int ITEMS, int NB, bool SELF = false>
 AbKernel<double> dmma_kernel_mt(int mtw) {
     switch (mtw) {
-        case 1: return k_sigma_ab_dmma<1, ITEMS, NB>;
-        case 2: return k_sigma_ab_dmma<2, ITEMS, NB>;
-        case 3: return k_sigma_ab_dmma<3, ITEMS, NB>;
-        case 4: return k_sigma_ab_dmma<4, ITEMS, NB>;
-        case 5: return k_sigma_ab_dmma<5, ITEMS, NB>;
-        case 6: return k_sigma_ab_dmma<6, ITEMS, NB>;
-        case 7: return k_sigma_ab_dmma<7, ITEMS, NB>;
-        case 8: return k_sigma_ab_dmma<8, ITEMS, NB>;
-        case 9: return k_sigma_ab_dmma<9, ITEMS, NB>;
+        case 1: return k_sigma_ab_dmma<1, ITEMS, NB, SELF>;
+        case 2: return k_sigma_ab_dmma<2, ITEMS, NB, SELF>;
+        case 3: return k_sigma_ab_dmma<3, ITEMS, NB, SELF>;
+        case 4: return k_sigma_ab_dmma<4, ITEMS, NB, SELF>;
+        case 5: return k_sigma_ab_dmma<5, ITEMS, NB, SELF>;
+        case 6: return k_sigma_ab_dmma<6, ITEMS, NB, SELF>;
+        case 7: return k_sigma_ab_dmma<7, ITEMS, NB, SELF>;
+        case 8: return k_sigma_ab_dmma<8, ITEMS, NB, SELF>;
+        case 9: return k_sigma_ab_dmma<9, ITEMS, NB, SELF>;
         default: return nullptr;
     }
 }
 
-template <int ITEMS, int NB, int AS>
+template <int ITEMS, int NB, int AS, bool SELF = false>
 AbKernel<float> tf32_kernel_mt(int mt) {
     switch (mt) {
-        case 1: return k_sigma_ab_tf32<1, ITEMS, NB, AS>;
-        case 2: return k_sigma_ab_tf32<2, ITEMS, NB, AS>;
-        case 3: return k_sigma_ab_tf32<3, ITEMS, NB, AS>;
-        case 4: return k_sigma_ab_tf32<4, ITEMS, NB, AS>;
-        case 5: return k_sigma_ab_tf32<5, ITEMS, NB, AS>;
+        case 1: return k_sigma_ab_tf32<1, ITEMS, NB, AS, SELF>;
+        case 2: return k_sigma_ab_tf32<2, ITEMS, NB, AS, SELF>;
+        case 3: return k_sigma_ab_tf32<3, ITEMS, NB, AS, SELF>;
+        case 4: return k_sigma_ab_tf32<4, ITEMS, NB, AS, SELF>;
+        case 5: return k_sigma_ab_tf32<5, ITEMS, NB, AS, SELF>;
         default: return nullptr;
     }
 }
@@ -624,12 +645,17 @@ bool use_dmma(int tx, size_t w) { return tx == 16 && w == sizeof(double); }
 bool use_tf32(int tx, size_t w) { return tx == 16 && w == sizeof(float); }
 
 template <typename T>
-AbKernel<T> ab_kernel(int tx, int mrows, int items, int nbuf) {
+AbKernel<T> ab_kernel(int tx, int mrows, int items, int nbuf, bool self) {
+    if (self && items != 4) return nullptr;  // not asked for (ab_self)
     if constexpr (sizeof(T) == sizeof(float)) {
         if (use_tf32(tx, sizeof(T))) {
             // variant 3: one B buffer and the A panel pre-split; 1: one B
             // buffer; 2: two B buffers
             const int mt = tf_mt(mrows);
+            if (self)
+                return nbuf == 3   ? tf32_kernel_mt<4, 1, 1, true>(mt)
+                       : nbuf == 1 ? tf32_kernel_mt<4, 1, 0, true>(mt)
+                                   : tf32_kernel_mt<4, 2, 0, true>(mt);
             if (nbuf == 3)
                 return items == 4 ? tf32_kernel_mt<4, 1, 1>(mt) : tf32_kernel_mt<16, 1, 1>(mt);
             if (nbuf == 1)
@@ -640,6 +666,9 @@ AbKernel<T> ab_kernel(int tx, int mrows, int items, int nbuf) {
     if constexpr (sizeof(T) == sizeof(double)) {
         if (use_dmma(tx, sizeof(T))) {
             const int mtw = dm_mtw(mrows);
+            if (self)
+                return nbuf == 1 ? dmma_kernel_mt<4, 1, true>(mtw)
+                                 : dmma_kernel_mt<4, 2, true>(mtw);
             if (nbuf == 1)
                 return items == 4 ? dmma_kernel_mt<4, 1>(mtw) : dmma_kernel_mt<16, 1>(mtw);
             return items == 4 ? dmma_kernel_mt<4, 2>(mtw) : dmma_kernel_mt<16, 2>(mtw);
@@ -696,6 +725,22 @@ bool ab_possible(const AbShape &sh, int tx, size_t w, size_t smem_max) {
         return false;
     }
     return ab_smem(sh, tx, w) <= smem_max;
+}
+
+// Whether the product takes the string itself as one more column (jself):
+// where that column fills a padded k step, or where a launch costs more than a
+// k step.  Measured, a whole sigma (us, with k_coulomb -> with jself): FP64 31
+// columns in 32 at 213 444 determinants 145 -> 134, 26 in 28 at 63 504 47 -> 41,
+// 17 in 20 at 4 900 29 -> 24; FP32 26 in 32 at 63 504 42 -> 36; where it is not
+// taken, FP64 37 in 40 at 853 776 488 -> 491, at 511 225 364 -> 392.
+bool ab_self(const AbShape &sh, long long ndets, int tx, size_t w, size_t smem_max) {
+    AbShape more = sh;
+    more.sa++;
+    if ((!use_tf32(tx, w) && !use_dmma(tx, w)) || ab_items(sh.nb) != 4) return false;
+    const bool fits = use_tf32(tx, w) ? tf_k8(more.sa) == tf_k8(sh.sa)
+                                      : dm_k4(more.sa) == dm_k4(sh.sa);
+    return (fits || ndets <= 65536) && ab_possible(sh, tx, w, smem_max) &&
+           ab_smem(more, tx, w) <= smem_max;
 }
 
 // Per-chunk entry lists of the beta side (see the header comment): for
@@ -795,9 +840,9 @@ jci_status ab_launch(const AbArgs<T> &a, int tx, int device, const T *v, T *o,
     for (int nbuf : {3, 1, 2}) {
         if (nbuf == 3 && !use_tf32(tx, sizeof(T))) continue;
         if (nbuf == 1 && !use_dmma(tx, sizeof(T)) && !use_tf32(tx, sizeof(T))) continue;
-        kern = ab_kernel<T>(tx, a.mrows, items, nbuf);
+        kern = ab_kernel<T>(tx, a.mrows, items, nbuf, a.jself != nullptr);
         if (!kern) return JCI_ERR_SPACE;
-        smem = ab_smem_bytes(tx, sizeof(T), a.sa, a.mrows, nbuf, a.maxent, a.offs);
+        smem = ab_smem_bytes(tx, sizeof(T), a.sa + (a.jself ? 1 : 0), a.mrows, nbuf, a.maxent, a.offs);
         JCI_CUDA(smem_optin(kern));
         JCI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kAbThreads, smem));
         if (nbuf == 2 || occ >= 2) break;

@@ -11,7 +11,7 @@
 // FP64 tensor cores (mma.sync m8n8k4) with operands from shared memory, while
 // the list kernels wait on a table load for every term.  FP32 operands are
 // widened, so its sums are exact to FP64.  Measured, FP64, against the row
-// kernel: 126 strings of each spin 10 us for 44, 252 17 for 66, 924 142 for 512
+// kernel: 126 strings of each spin 10 us for 44, 252 16 for 66, 924 142 for 512
 // (group kernel, transposes and stream of plan 7 there: 240); the tensor cores
 // alone would take 85 of the 142.
 #include <cuda_pipeline.h>
@@ -26,14 +26,13 @@ namespace jci {
 namespace {
 
 constexpr int kDPad = 32;         // rows of H are padded to this
-constexpr int kDThreads = 128;    // 2 x 2 warps
 constexpr int kDFlush = 128;      // k per partial sum
 
 constexpr int kDKC = 32;          // k per staged chunk
 
 // Chunks in flight: two leave room for three CTAs of the widest tile per SM
 // (four of 16 measured the same: 142 to 150 us at FCI(12,12)).
-__host__ __device__ constexpr int dense_stages(int mt) { return mt == 4 ? 2 : 3; }
+__host__ __device__ constexpr int dense_stages(int bm) { return bm == 64 ? 2 : 3; }
 
 template <typename T>
 struct DenseArgs {
@@ -71,15 +70,17 @@ __device__ __noinline__ double dense_linked(const DenseArgs<T> &a, const T *C, i
     return sum;
 }
 
-// Output tile 16 MT x 16 NT: each of the 2 x 2 warps 8 MT x 8 NT; k runs over
+// Output tile 8 MT WM x 16 NT: each of the WM x 2 warps 8 MT x 8 NT; k runs over
 // the alpha strings (A = H_alpha, B = C), then the beta strings (A = C,
-// B = H_beta), chunks double-buffered with cp.async.
-template <typename T, int MT, int NT>
-__global__ void __launch_bounds__(kDThreads)
+// B = H_beta), chunks pipelined with cp.async.  32 x 32 tiles take eight warps
+// (462 strings 36 us, 40 with four), 64 x 32 tiles four (924 strings 142 us, 146
+// with eight).
+template <typename T, int MT, int NT, int WM>
+__global__ void __launch_bounds__(64 * WM)
     k_same_dense(DenseArgs<T> a, const T *__restrict__ C, T *__restrict__ S) {
     if (a.skip && *a.skip) return;
-    constexpr int BM = 16 * MT, BN = 16 * NT, AS = kDAS, BS = kDBS<T, BN>;
-    constexpr int KC = kDKC, ST = dense_stages(MT);
+    constexpr int NTH = 64 * WM, BM = 8 * MT * WM, BN = 16 * NT, AS = kDAS, BS = kDBS<T, BN>;
+    constexpr int KC = kDKC, ST = dense_stages(BM);
     constexpr int VE = 16 / sizeof(T);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *As = reinterpret_cast<T *>(smem_raw);   // [ST][BM][AS]
@@ -94,7 +95,7 @@ __global__ void __launch_bounds__(kDThreads)
                     int len, long long ld, bool vec) {
         if (vec) {
             const int per = cols / VE;
-            for (int idx = tid; idx < rows * per; idx += kDThreads) {
+            for (int idx = tid; idx < rows * per; idx += NTH) {
                 const int r = idx / per, c = VE * (idx - r * per);
                 T *d = dst + r * stride + c;
                 if (r0 + r < nr && c0 + c < len)  // len is a multiple of VE
@@ -103,7 +104,7 @@ __global__ void __launch_bounds__(kDThreads)
                     *reinterpret_cast<uint4 *>(d) = make_uint4(0, 0, 0, 0);
             }
         } else {
-            for (int idx = tid; idx < rows * cols; idx += kDThreads) {
+            for (int idx = tid; idx < rows * cols; idx += NTH) {
                 const int r = idx / cols, c = idx - r * cols;
                 T *d = dst + r * stride + c;
                 if (r0 + r < nr && c0 + c < len)
@@ -218,14 +219,14 @@ __global__ void __launch_bounds__(128)
     }
 }
 
-template <typename T, int MT, int NT>
+template <typename T, int MT, int NT, int WM>
 jci_status dense_launch_t(const DenseArgs<T> &a, const T *x, T *y, cudaStream_t st) {
-    constexpr int BM = 16 * MT, BN = 16 * NT;
-    const size_t smem = dense_stages(MT) *
+    constexpr int BM = 8 * MT * WM, BN = 16 * NT;
+    const size_t smem = dense_stages(BM) *
                         (size_t)(BM * kDAS + kDKC * kDBS<T, BN>) * sizeof(T);
-    JCI_CUDA(smem_optin(k_same_dense<T, MT, NT>));
+    JCI_CUDA(smem_optin(k_same_dense<T, MT, NT, WM>));
     dim3 g((a.nb + BN - 1) / BN, (a.na + BM - 1) / BM);
-    k_same_dense<T, MT, NT><<<g, kDThreads, smem, st>>>(a, x, y);
+    k_same_dense<T, MT, NT, WM><<<g, 64 * WM, smem, st>>>(a, x, y);
     JCI_CUDA(cudaGetLastError());
     return JCI_OK;
 }
@@ -285,9 +286,9 @@ jci_status same_dense_launch(const SameDense &t, const T *hd, const int *skip, i
     auto ctas = [&](int bm, int bn) {
         return (long long)((a.na + bm - 1) / bm) * ((a.nb + bn - 1) / bn);
     };
-    if (ctas(64, 32) >= 2 * nsm) return dense_launch_t<T, 4, 2>(a, x, y, st);
-    if (ctas(32, 32) >= nsm) return dense_launch_t<T, 2, 2>(a, x, y, st);
-    return dense_launch_t<T, 1, 2>(a, x, y, st);
+    if (ctas(64, 32) >= 2 * nsm) return dense_launch_t<T, 4, 2, 2>(a, x, y, st);
+    if (ctas(32, 32) >= nsm) return dense_launch_t<T, 1, 2, 4>(a, x, y, st);
+    return dense_launch_t<T, 1, 2, 2>(a, x, y, st);
 }
 
 template jci_status same_dense_launch<double>(const SameDense &, const double *, const int *, int,

@@ -45,6 +45,7 @@ struct AbArgs {
     const uint32_t *base;   // [chunk + 1] first entry of each chunk (multiples of 4)
     const uint32_t *ent;    // col | row << 8 | phase << 31
     const int *skip;        // nonzero: return at once
+    const T *jself;         // [pair][Ia] sum_{m in Ia} (mm|pair), or null; with it S is set
 };
 struct AbTables {
     int tx = 0, nchunk = 0, offs = 0, maxent = 0;
@@ -56,6 +57,7 @@ struct AbShape {
 };
 size_t ab_smem(const AbShape &sh, int tx, size_t w);
 bool ab_possible(const AbShape &sh, int tx, size_t w, size_t smem_max);
+bool ab_self(const AbShape &sh, long long ndets, int tx, size_t w, size_t smem_max);
 jci_status ab_tables_build(const jci_space *s, int npair, int tx, AbTables *t);
 void ab_tables_free(AbTables *t);
 template <typename T>
