@@ -495,9 +495,14 @@ static jci_status dense_fill(jci_space *s) {
     cudaStream_t st = d->stream;
     d->dense_ld = ((int)s->ndets + 31) / 32 * 32;
     const size_t n = (size_t)s->ndets * d->dense_ld;
-    if (!d->dense) {
-        JCI_CUDA(cudaMalloc(&d->densef, n * sizeof(float)));
-        JCI_CUDA(cudaMalloc(&d->dense, n * sizeof(double)));
+    if (!d->dense &&
+        (cudaMalloc(&d->densef, n * sizeof(float)) != cudaSuccess ||
+         cudaMalloc(&d->dense, n * sizeof(double)) != cudaSuccess)) {
+        cudaGetLastError();  // without room for H the space takes its other path
+        cudaFree(d->densef);
+        d->densef = nullptr;
+        d->dense = nullptr;
+        return JCI_OK;
     }
     JCI_CUDA(cudaMemsetAsync(d->dense, 0, n * sizeof(double), st));
     JCI_CUDA(cudaMemsetAsync(d->densef, 0, n * sizeof(float), st));

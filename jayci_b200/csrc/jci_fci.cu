@@ -2360,6 +2360,7 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
     DeviceState *d = s->dev;
     FciTables *f = d->fci;
     const int prec = sizeof(T) == 8 ? 0 : 1;
+    const bool sd_kept = f->sd_state == 1;
     size_t w = sizeof(T);
     long long n = (long long)f->na * f->nb;
     T *v = nullptr, *o = nullptr;
@@ -2621,9 +2622,9 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
         group_tables_free(&f->grp[0]);
         group_tables_free(&f->grp[1]);
     }
-    // nor the same-spin matrices
-    if (!dense && f->sd_state == 1 &&
-        !(f->tuned_mode[prec ^ 1] == 5 && f->tuned_nt[prec ^ 1] == kSplitSingles)) {
+    // nor the same-spin matrices, unless an earlier plan (and what was captured
+    // of it) uses them
+    if (!dense && !sd_kept && f->sd_state == 1) {
         same_dense_free(&f->sd);
         f->sd_state = 0;
     }
