@@ -153,10 +153,19 @@ def profile_key(mode, R, B, nt=None):
     column blocks (16 <= R < 32), ":row" when one panel per alpha row is
     shared by all CTAs (32 <= R < 64), ":cp" for the compact panel (R >= 64);
     ":hs" after the group variant when the beta singles run through hole
-    strings (nt = 0)."""
+    strings (nt = 0), ":split" when the singles are split between the hole
+    strings and the Coulomb pass (nt = 1); "5:sd" for dense same-spin
+    products (nt = 1); ":i8" for the integer-digit product with another row
+    or stream plan."""
     key = f"{mode}:{B}" if mode in (6, 7) else str(mode)
     if mode in (6, 7) and nt == 0:
         key += ":hs"
+    if mode in (6, 7) and nt == 1:
+        return key + ":split"
+    if mode == 5 and nt == 1:
+        key += ":sd"
+    if mode in (4, 5, 7) and R == 128:
+        key += ":i8"
     if mode in (1, 3, 6) and R >= 64:
         key += ":cp"
     elif mode in (1, 3, 6) and R >= 32:
