@@ -14,10 +14,11 @@
 //   Y[I][c]    = sum_{K in I} E[K][I - K][c]          (phase 2, C(N,2) rows)
 // At FCI(16,16): 8008 hole strings with 45 pairs each (1260 of the 2025
 // block entries are doubles), against the string-group form's 16 x 3.7
-// reached rows per union entry.  Phase 1 runs in FP64 on the FP64 tensor
-// cores (mma.sync m8n8k4) and in FP32 on the FMA pipes; E is kept for one
-// block of columns at a time.  Every sum runs in a fixed order: bitwise
-// reproducible.
+// reached rows per union entry.  Phase 1 runs on the FP64 tensor cores
+// (mma.sync m8n8k4) with W_K in registers, FP32 operands widened
+// (k_pairs_mma; more than 80 pairs per hole string: k_pairs_product); E is
+// kept for one block of columns at a time.  Every sum runs in a fixed order:
+// bitwise reproducible.
 #include <cuda_pipeline.h>
 
 #include <algorithm>
