@@ -239,7 +239,9 @@ jci_status jci_sigma_tuning(const jci_space *s, int precision, int *mode,
 
 /* Fix the sigma plan instead of autotuning (for tests and measurements),
  * with the mode and arguments as jci_sigma_tuning reports them; threads =
- * 128/256/512/1024 per CTA.  Only for one-group (FCI/CAS) spaces after
+ * 128/256/512/1024 per CTA where it counts threads.  All 0, which
+ * jci_sigma_tuning reports for a space of at most 2048 determinants, is its
+ * one dense product.  Only for one-group (FCI/CAS) spaces after
  * jci_set_integrals; JCI_ERR_ARG for a plan the space cannot run.  No
  * reference counterpart. */
 jci_status jci_sigma_set_plan(jci_space *s, int precision, int mode,

@@ -50,7 +50,7 @@ struct FciTables {
     bool tuned[2] = {false, false};                 // per precision (autotuned)
     bool forced[2] = {false, false};                // fixed by the caller
     int tuned_nt[2] = {0, 0}, tuned_R[2] = {0, 0};
-    int tuned_mode[2] = {0, 0}, tuned_B[2] = {1, 1};
+    int tuned_mode[2] = {0, 0}, tuned_B[2] = {0, 0};
     float tuned_ms[2] = {0.f, 0.f};
     int mix_grid[2] = {0, 0};      // resident CTAs of k_sigma_mixed
     int mix_occ[2] = {1, 1}, nsm = 0;
@@ -1512,11 +1512,11 @@ static jci_status launch_rows(const FciArgs<T> &a, int nt, int RB, const T *v, T
 }
 
 static bool rows_ok(int nb, int nt, int RB) {
+    if (nt != 128 && nt != 256 && nt != 512 && nt != 1024) return false;
     int items = (nb + nt - 1) / nt;
     int IT = items <= 2 ? 2 : items <= 4 ? 4 : items <= 8 ? 8 : items <= 16 ? 16 : 32;
     if (items > 32 || IT * RB > 32) return false;
     if (RB != 1 && RB != 2 && RB != 4) return false;
-    if (nt != 128 && nt != 256 && nt != 512 && nt != 1024) return false;
     return nt <= (IT * RB <= 4 ? 1024 : 512);
 }
 
@@ -2717,6 +2717,14 @@ jci_status fci_force_plan(jci_space *s, int precision, int mode, int nt, int R, 
     if (!f) return JCI_ERR_STATE;
     int p = precision == JCI_FP32 ? 1 : 0;
     size_t w = p ? sizeof(float) : sizeof(double);
+    if (mode == 0 && nt == 0 && R == 0 && (B == 0 || B == 1)) {
+        // what fci_tuning reports where sigma is the one dense product
+        if (!s->dev->dense) return JCI_ERR_ARG;
+        f->tuned[p] = f->forced[p] = false;
+        f->tuned_mode[p] = f->tuned_nt[p] = f->tuned_R[p] = f->tuned_B[p] = 0;
+        f->tuned_ms[p] = 0.f;
+        return JCI_OK;
+    }
     if (mode == 6 || mode == 7) {
         bool ok = mode == 6 ? mixed_possible(f, w) && R >= 0 : ab_plan_possible(s, R, w, s->dev->stream);
         bool ok1 = true;
@@ -2744,10 +2752,9 @@ jci_status fci_force_plan(jci_space *s, int precision, int mode, int nt, int R, 
         } else if (!ok || !rows_ok(f->nb, nt, B) || rows_smem(f->nb, f->npair, f->da, B, w) > f->smem_max)
             return JCI_ERR_ARG;
     } else {
+        if (nt != 128 && nt != 256 && nt != 512 && nt != 1024) return JCI_ERR_ARG;
         int items = (f->nb + nt - 1) / nt;
-        if ((nt != 128 && nt != 256 && nt != 512 && nt != 1024) || items > 32 ||
-            (nt == 1024 && items > 2))
-            return JCI_ERR_ARG;
+        if (items > 32 || (nt == 1024 && items > 2)) return JCI_ERR_ARG;
         if (R < 1 || fci_smem(f->nb, f->npair, R, w) > f->smem_max) return JCI_ERR_ARG;
     }
     if (mode == 4 || mode == 5 || mode == 7) {  // tables are built here, outside any capture
