@@ -2712,9 +2712,8 @@ bool fci_forced(const jci_space *s, int precision) {
     return f && f->forced[precision == JCI_FP32 ? 1 : 0];
 }
 
-jci_status fci_force_plan(jci_space *s, int precision, int mode, int nt, int R, int B) {
-    FciTables *f = s->dev ? s->dev->fci : nullptr;
-    if (!f) return JCI_ERR_STATE;
+static jci_status force_plan(jci_space *s, int precision, int mode, int nt, int R, int B) {
+    FciTables *f = s->dev->fci;
     int p = precision == JCI_FP32 ? 1 : 0;
     size_t w = p ? sizeof(float) : sizeof(double);
     if (mode == 0 && nt == 0 && R == 0 && (B == 0 || B == 1)) {
@@ -2785,6 +2784,15 @@ jci_status fci_force_plan(jci_space *s, int precision, int mode, int nt, int R, 
     f->tuned_B[p] = mode != 0 ? B : 1;
     f->tuned_ms[p] = 0.f;
     return JCI_OK;
+}
+
+jci_status fci_force_plan(jci_space *s, int precision, int mode, int nt, int R, int B) {
+    if (!s->dev || !s->dev->fci) return JCI_ERR_STATE;
+    const jci_status r = force_plan(s, precision, mode, nt, R, B);
+    // A plan's tables are filled by kernels and copies on the handle's stream
+    // (a refused plan leaves some too); the first sigma may run on another.
+    JCI_CUDA(cudaStreamSynchronize(s->dev->stream));
+    return r;
 }
 
 // ---- allocation-free sigma ----------------------------------------------
