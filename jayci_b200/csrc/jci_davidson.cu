@@ -80,7 +80,7 @@ struct DavidsonBuffers {
     int *info = nullptr;         // status word of k_jacobi
     cudaGraphExec_t gexec[2] = {nullptr, nullptr};  // FP64, FP32 sigma
     int gkmax[2] = {0, 0};
-    int gplan[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+    int ggen[2][2] = {{0, 0}, {0, 0}};
 };
 
 static void drop_graphs(DavidsonBuffers *b) {
@@ -1082,17 +1082,13 @@ static jci_status enqueue_iteration(Ctx &c, bool fp32, int kmax) {
     return JCI_OK;
 }
 
-// Capture (once per precision, basis size and sigma plan) the iteration as
-// a CUDA graph.  The sigma kernels see the control block's stop flag.
+// Capture (once per precision, basis size and state of sigma's plans and
+// scratch) the iteration as a CUDA graph.  The sigma kernels see the control block's stop flag.
 static jci_status ensure_graph(Ctx &c, bool fp32, int kmax) {
     DavidsonBuffers *b = c.b;
     const int p = fp32 ? 1 : 0;
-    int plan[4] = {0, 0, 0, 0};
-    if (c.d->fci) {
-        float ms = 0.f;
-        fci_tuning(c.s, fp32 ? JCI_FP32 : JCI_FP64, &plan[0], &plan[1], &plan[2], &plan[3], &ms);
-    }
-    if (b->gexec[p] && b->gkmax[p] == kmax && memcmp(plan, b->gplan[p], sizeof plan) == 0)
+    const int gen[2] = {c.d->sigma_gen, embed_generation(c.d)};
+    if (b->gexec[p] && b->gkmax[p] == kmax && memcmp(gen, b->ggen[p], sizeof gen) == 0)
         return JCI_OK;
     if (b->gexec[p]) {
         cudaGraphExecDestroy(b->gexec[p]);
@@ -1118,7 +1114,7 @@ static jci_status ensure_graph(Ctx &c, bool fp32, int kmax) {
     cudaGetLastError();
     if (r) return r;
     b->gkmax[p] = kmax;
-    memcpy(b->gplan[p], plan, sizeof plan);
+    memcpy(b->ggen[p], gen, sizeof gen);
     return JCI_OK;
 }
 

@@ -92,6 +92,9 @@ struct DeviceState {
     // into a CUDA graph, so that iterations launched after the solve has
     // stopped cost no sigma work; null otherwise.
     const int *sigma_skip = nullptr;
+    // Counts the times that sigma's plan, route or scratch changed: a captured
+    // sigma holds their addresses and serves one value only.
+    int sigma_gen = 0;
 };
 
 // Kernel-facing view of a space (POD, passed by value).

@@ -86,6 +86,10 @@ void embed_free(DeviceState *d) {
     d->emb = nullptr;
 }
 
+int embed_generation(const DeviceState *d) {
+    return d->emb && d->emb->full && d->emb->full->dev ? d->emb->full->dev->sigma_gen : 0;
+}
+
 jci_status embed_wait_status(const DeviceState *d) {
     return d->emb && d->emb->full ? fci_wait_status(d->emb->full) : JCI_OK;
 }
@@ -236,6 +240,7 @@ bool embed_chosen(jci_space *s, const void *v, void *o, long long ld, int precis
         e->use[prec] = 1;
         return true;
     }
+    d->sigma_gen++;
     cudaFree(e->v[prec]);
     cudaFree(e->o[prec]);
     e->v[prec] = e->o[prec] = nullptr;

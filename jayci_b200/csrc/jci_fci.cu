@@ -2078,6 +2078,7 @@ static jci_status launch_hs(jci_space *s, const StreamArgs<T> &be, const T *ct, 
         JCI_CUDA(cudaStreamIsCapturing(st, &cs));
         if (cs != cudaStreamCaptureStatusNone) return JCI_ERR_STATE;
         JCI_CUDA(cudaFree(f->hbuf[prec]));
+        s->dev->sigma_gen++;
         f->hbuf[prec] = nullptr;
         f->hbytes[prec] = 0;
         JCI_CUDA(cudaMalloc(&f->hbuf[prec], need));
@@ -2105,6 +2106,7 @@ static jci_status pair_scratch(jci_space *s, int items, cudaStream_t st, T **E) 
         JCI_CUDA(cudaStreamIsCapturing(st, &cs));
         if (cs != cudaStreamCaptureStatusNone) return JCI_ERR_STATE;
         JCI_CUDA(cudaFree(f->pbuf[prec]));
+        s->dev->sigma_gen++;
         f->pbuf[prec] = nullptr;
         f->pbytes[prec] = 0;
         JCI_CUDA(cudaMalloc(&f->pbuf[prec], need));
@@ -2610,6 +2612,7 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
         b1B = 1;
     }
     const bool streams = mode == 3 || mode == 4, groups = mode == 6 || mode == 7;
+    d->sigma_gen++;
     f->tuned[prec] = true;
     f->tuned_mode[prec] = mode;
     f->tuned_nt[prec] = groups ? b6s : streams ? b3a : mode ? b1nt : b0nt;
@@ -2789,6 +2792,7 @@ static jci_status force_plan(jci_space *s, int precision, int mode, int nt, int 
 jci_status fci_force_plan(jci_space *s, int precision, int mode, int nt, int R, int B) {
     if (!s->dev || !s->dev->fci) return JCI_ERR_STATE;
     const jci_status r = force_plan(s, precision, mode, nt, R, B);
+    s->dev->sigma_gen++;
     // A plan's tables are filled by kernels and copies on the handle's stream
     // (a refused plan leaves some too); the first sigma may run on another.
     JCI_CUDA(cudaStreamSynchronize(s->dev->stream));

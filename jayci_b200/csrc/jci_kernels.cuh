@@ -207,6 +207,7 @@ bool embed_chosen(jci_space *s, const void *v, void *o, long long ld, int precis
                   cudaStream_t st);
 jci_status embed_sigma(jci_space *s, int nvec, const void *v, void *o, long long ld, int precision,
                        cudaStream_t st);
+int embed_generation(const DeviceState *d);
 jci_status embed_set_integrals(jci_space *s);
 jci_status embed_wait_status(const DeviceState *d);
 void embed_free(DeviceState *d);
