@@ -247,6 +247,27 @@ jci_status jci_sigma_tuning(const jci_space *s, int precision, int *mode,
 jci_status jci_sigma_set_plan(jci_space *s, int precision, int mode,
                               int threads, int rows, int batch);
 
+/* How sigma of a space with several occupation groups per spin runs: *route
+ * is 1 for the generic kernel, 2 for the full CI space of the same electrons
+ * and orbitals, of which sigma is a diagonal block; then mode, threads, rows
+ * and batch are the full space's plan as jci_sigma_tuning reports it.  The
+ * first sigma of a precision times both where both can run, so two processes
+ * may take different ones and agree to rounding only.  All 0 before that
+ * sigma, for one-group spaces, and where sigma is one dense product (at most
+ * 2048 determinants).  No reference counterpart. */
+jci_status jci_sigma_route(const jci_space *s, int precision, int *route,
+                           int *mode, int *threads, int *rows, int *batch);
+
+/* Fix the route with the values that jci_sigma_route reports, after
+ * jci_set_integrals: 0 times both at the next sigma, 1 and 2 as above (2 with
+ * mode to batch all 0 leaves the full space's plan to its autotuner).  Waits
+ * for the device.  JCI_ERR_ARG for a route that the space does not have:
+ * the full space is for spaces of at least 16384 determinants whose full
+ * space has at most 16 times as many and 16384 strings of a spin, while its
+ * memory fits.  No reference counterpart. */
+jci_status jci_sigma_set_route(jci_space *s, int precision, int route, int mode,
+                               int threads, int rows, int batch);
+
 /* Test hook for the device-side wait bounds.  The next sigma whose product
  * runs through the row panels shared by all CTAs (plan rows >= 32) leaves
  * the panel work of its first two alpha rows undone, so the gathers that

@@ -109,6 +109,8 @@ def lib():
                                        ctypes.POINTER(ip), ctypes.POINTER(ip),
                                        ctypes.POINTER(ctypes.c_float)]
         L.jci_sigma_set_plan.argtypes = [vp, ip, ip, ip, ip, ip]
+        L.jci_sigma_route.argtypes = [vp, ip] + [ctypes.POINTER(ip)] * 5
+        L.jci_sigma_set_route.argtypes = [vp, ip, ip, ip, ip, ip, ip]
         L.jci_read_namelists.argtypes = [ctypes.c_char_p, vp, vp, vp]
         L.jci_read_moints.argtypes = [ctypes.c_char_p, vp, ctypes.c_longlong, vp,
                                       ctypes.c_longlong, ctypes.POINTER(ip),
@@ -243,6 +245,19 @@ class Space:
         """Fix the FCI sigma plan (modes 0-7 of jci_sigma_set_plan)."""
         _check(lib().jci_sigma_set_plan(self.h, precision, mode, threads, rows, batch),
                "sigma_set_plan")
+
+    def sigma_route(self, precision=FP64):
+        """(route, mode, threads, rows, batch) of a space with several
+        occupation groups, with the meanings of jci_sigma_route."""
+        x = [ctypes.c_int() for _ in range(5)]
+        _check(lib().jci_sigma_route(self.h, precision, *[ctypes.byref(k) for k in x]),
+               "sigma_route")
+        return tuple(k.value for k in x)
+
+    def set_sigma_route(self, precision, route, mode=0, threads=0, rows=0, batch=0):
+        """Fix the route of sigma (jci_sigma_set_route)."""
+        _check(lib().jci_sigma_set_route(self.h, precision, route, mode, threads, rows, batch),
+               "sigma_set_route")
 
     def davidson(self, maxiter=500, krymin=4, krymax=12, nroots=1, prediagr=1,
                  refdim=8, restol=1e-8, precision=FP64, switch_tol=1e-4,

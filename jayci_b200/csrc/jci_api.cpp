@@ -163,6 +163,29 @@ jci_status jci_sigma_set_plan(jci_space *s, int precision, int mode, int threads
     return fci_force_plan(s, precision, mode, threads, rows, batch);
 }
 
+// 0: one route only (one group per spin: see the plans; or one dense product)
+static bool routed(const jci_space *s) { return s->dev && !s->dev->single_group && !s->dev->dense; }
+
+jci_status jci_sigma_route(const jci_space *s, int precision, int *route, int *mode, int *threads,
+                           int *rows, int *batch) {
+    if (!s || !route || !mode || !threads || !rows || !batch) return JCI_ERR_ARG;
+    if (precision != JCI_FP64 && precision != JCI_FP32) return JCI_ERR_ARG;
+    *route = *mode = *threads = *rows = *batch = 0;
+    if (routed(s)) embed_route(s->dev, precision, route, mode, threads, rows, batch);
+    return JCI_OK;
+}
+
+jci_status jci_sigma_set_route(jci_space *s, int precision, int route, int mode, int threads,
+                               int rows, int batch) {
+    if (!s || (precision != JCI_FP64 && precision != JCI_FP32)) return JCI_ERR_ARG;
+    if (route < kRouteTimed || route > kRouteFull) return JCI_ERR_ARG;
+    if (route != kRouteFull && (mode || threads || rows || batch)) return JCI_ERR_ARG;
+    if (mode < 0 || mode > 7) return JCI_ERR_ARG;
+    if (!s->have_ints) return JCI_ERR_STATE;
+    if (!routed(s)) return route == kRouteTimed ? JCI_OK : JCI_ERR_ARG;
+    return embed_set_route(s, precision, route, mode, threads, rows, batch);
+}
+
 jci_status jci_test_expire_next_wait(jci_space *s) {
     if (!s) return JCI_ERR_ARG;
     if (!s->have_ints || !fci_supported(s)) return JCI_ERR_STATE;

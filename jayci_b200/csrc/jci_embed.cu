@@ -10,7 +10,9 @@
 // and gathers single elements.  It pays while the full space is not too many
 // times larger: measured per determinant, the generic kernel takes 5 to 17 ns
 // and a full-space plan 0.4 to 0.8 ns, so up to kEmbedRatio = 16 the two are
-// timed once per precision and space, and the faster one is kept.
+// timed once per precision and space, and the faster one is kept.  The two sum
+// in different orders; a caller that needs the same bits in every process
+// reads the route and pins it (embed_route, embed_set_route).
 // Measured: 12 electrons in 16 orbitals (2 DOCC, 10 active, 4 virtual,
 // excitation level 2; 13.0 of 64.1 million determinants) FP64 215 -> 45.3 ms,
 // FP32 188 -> 32.2; 11 electrons in 15 orbitals (2 DOCC, 9 active; 3.2 of 15.0
@@ -34,7 +36,7 @@ struct Embedding {
     jci_space *full = nullptr;
     int *inv[2] = {nullptr, nullptr};   // [full string] string of the space, or -1
     void *v[2] = {nullptr, nullptr}, *o[2] = {nullptr, nullptr};  // full vectors, per precision
-    int use[2] = {0, 0};                // per precision: 0 not timed, 1 faster, -1 slower
+    int use[2] = {0, 0};                // per precision: 0 not timed, 1 this way, -1 the generic one
     bool none = false;                  // the space has no usable full space
 };
 
@@ -109,14 +111,12 @@ jci_status embed_set_integrals(jci_space *s) {
     return e && e->full ? embed_integrals(s) : JCI_OK;
 }
 
-// The full space and the string maps; false (and remembered) when there is
-// none within the limits or the device's free memory.
+// The full space and the string maps; false when there is none within the
+// limits or the device's free memory.
 static bool embed_build(jci_space *s) {
     DeviceState *d = s->dev;
     Embedding *e = d->emb;
     if (e->full) return true;
-    if (e->none) return false;
-    e->none = true;
     const int na = s->ci_aelec, nb = s->ci_belec, no = s->ci_orbs;
     if (s->ndets < kEmbedMin || no > 64 || na - nb < 0 || na - nb > 1) return false;
     const long long fa = binom(no, na), fb = binom(no, nb);
@@ -153,7 +153,6 @@ static bool embed_build(jci_space *s) {
         embed_drop(e);
         return false;
     }
-    e->none = false;
     return true;
 }
 
@@ -188,6 +187,27 @@ jci_status embed_sigma(jci_space *s, int nvec, const void *v, void *o, long long
     return embed_run<double>(s, nvec, (const double *)v, (double *)o, ld, st);
 }
 
+// Full-space vectors of one precision.
+static bool embed_vectors(Embedding *e, int prec) {
+    const size_t n = (size_t)e->full->sp[0].nstr * e->full->sp[1].nstr;
+    const size_t w = prec ? sizeof(float) : sizeof(double);
+    const bool ok = (e->v[prec] || cudaMalloc(&e->v[prec], n * w) == cudaSuccess) &&
+                    (e->o[prec] || cudaMalloc(&e->o[prec], n * w) == cudaSuccess);
+    if (!ok) cudaGetLastError();
+    return ok;
+}
+
+// A precision that does not come through here lets go of its vectors, and of
+// the full space when the other one does not either.
+static void embed_unused(DeviceState *d, int prec) {
+    Embedding *e = d->emb;
+    d->sigma_gen++;
+    cudaFree(e->v[prec]);
+    cudaFree(e->o[prec]);
+    e->v[prec] = e->o[prec] = nullptr;
+    if (e->use[0] < 0 && e->use[1] < 0) embed_drop(e);
+}
+
 // Whether sigma of this space runs through the full space; on the first call
 // of a precision (never while the stream is being captured) times one vector
 // both ways, on the caller's buffers.
@@ -197,19 +217,19 @@ bool embed_chosen(jci_space *s, const void *v, void *o, long long ld, int precis
     const int prec = precision == JCI_FP32 ? 1 : 0;
     if (!d->emb) d->emb = new (std::nothrow) Embedding();
     Embedding *e = d->emb;
-    if (!e || e->none) return false;
-    if (e->use[prec]) return e->use[prec] > 0;
+    if (!e) return false;
+    if (e->use[prec] || e->none) return e->use[prec] > 0;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
         return false;
-    if (!embed_build(s)) return false;
+    if (!embed_build(s)) {
+        e->none = true;
+        return false;
+    }
     e->use[prec] = -1;
-    const size_t n = (size_t)e->full->sp[0].nstr * e->full->sp[1].nstr;
-    const size_t w = prec ? sizeof(float) : sizeof(double);
     cudaEvent_t e0 = nullptr, e1 = nullptr;
-    bool ok = cudaMalloc(&e->v[prec], n * w) == cudaSuccess &&
-              cudaMalloc(&e->o[prec], n * w) == cudaSuccess &&
-              cudaEventCreate(&e0) == cudaSuccess && cudaEventCreate(&e1) == cudaSuccess;
+    bool ok = embed_vectors(e, prec) && cudaEventCreate(&e0) == cudaSuccess &&
+              cudaEventCreate(&e1) == cudaSuccess;
     const int *skip = d->sigma_skip;
     d->sigma_skip = nullptr;
     auto best = [&](auto fn) {
@@ -240,15 +260,48 @@ bool embed_chosen(jci_space *s, const void *v, void *o, long long ld, int precis
         e->use[prec] = 1;
         return true;
     }
-    d->sigma_gen++;
-    cudaFree(e->v[prec]);
-    cudaFree(e->o[prec]);
-    e->v[prec] = e->o[prec] = nullptr;
-    if (e->use[0] < 0 && e->use[1] < 0) {  // not used by either precision
-        embed_drop(e);
-        e->none = true;
-    }
+    embed_unused(d, prec);
     return false;
+}
+
+void embed_route(const DeviceState *d, int precision, int *route, int *mode, int *nt, int *R,
+                 int *B) {
+    const int prec = precision == JCI_FP32 ? 1 : 0;
+    const Embedding *e = d ? d->emb : nullptr;
+    float ms;
+    *route = *mode = *nt = *R = *B = 0;
+    if (!e) return;
+    // without a usable full space there is only the generic kernel
+    *route = e->use[prec] > 0 ? kRouteFull
+             : e->use[prec] < 0 || e->none ? kRouteGeneric : kRouteTimed;
+    if (*route == kRouteFull) fci_tuning(e->full, precision, mode, nt, R, B, &ms);
+}
+
+jci_status embed_set_route(jci_space *s, int precision, int route, int mode, int nt, int R, int B) {
+    DeviceState *d = s->dev;
+    const int prec = precision == JCI_FP32 ? 1 : 0;
+    if (!d->emb) d->emb = new (std::nothrow) Embedding();
+    Embedding *e = d->emb;
+    if (!e) return JCI_ERR_NOMEM;
+    JCI_CUDA(cudaDeviceSynchronize());  // nothing that is let go of is still in use
+    if (route == kRouteFull) {
+        if (!embed_build(s)) return JCI_ERR_ARG;
+        jci_status r = embed_vectors(e, prec) ? JCI_OK : JCI_ERR_NOMEM;
+        // all 0: the full space's own autotuner
+        if (!r && (mode || nt || R || B))
+            r = fci_force_plan(e->full, precision, mode, nt, R, B);
+        if (r) {
+            if (e->use[prec] <= 0) embed_unused(d, prec);
+            return r;
+        }
+        e->use[prec] = 1;
+        d->sigma_gen++;
+        return JCI_OK;
+    }
+    e->use[prec] = route == kRouteGeneric ? -1 : 0;
+    embed_unused(d, prec);
+    if (route == kRouteTimed) e->none = false;
+    return JCI_OK;
 }
 
 }  // namespace jci

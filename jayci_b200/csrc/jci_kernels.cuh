@@ -207,6 +207,12 @@ bool embed_chosen(jci_space *s, const void *v, void *o, long long ld, int precis
                   cudaStream_t st);
 jci_status embed_sigma(jci_space *s, int nvec, const void *v, void *o, long long ld, int precision,
                        cudaStream_t st);
+// The route that sigma of a truncated space takes, and the full space's plan;
+// which one it is to take, and with which plan (all 0: autotuned).
+constexpr int kRouteTimed = 0, kRouteGeneric = 1, kRouteFull = 2;
+void embed_route(const DeviceState *d, int precision, int *route, int *mode, int *nt, int *R,
+                 int *B);
+jci_status embed_set_route(jci_space *s, int precision, int route, int mode, int nt, int R, int B);
 int embed_generation(const DeviceState *d);
 jci_status embed_set_integrals(jci_space *s);
 jci_status embed_wait_status(const DeviceState *d);
