@@ -198,14 +198,14 @@ static bool embed_vectors(Embedding *e, int prec) {
 }
 
 // A precision that does not come through here lets go of its vectors, and of
-// the full space when the other one does not either.
+// the full space unless the other one does (a later precision builds it again).
 static void embed_unused(DeviceState *d, int prec) {
     Embedding *e = d->emb;
     d->sigma_gen++;
     cudaFree(e->v[prec]);
     cudaFree(e->o[prec]);
     e->v[prec] = e->o[prec] = nullptr;
-    if (e->use[0] < 0 && e->use[1] < 0) embed_drop(e);
+    if (e->use[prec ^ 1] <= 0) embed_drop(e);
 }
 
 // Whether sigma of this space runs through the full space; on the first call

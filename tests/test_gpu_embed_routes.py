@@ -104,3 +104,23 @@ def test_routes_refused():
         one.set_sigma_route(jb.FP64, 1)
     assert ei.value.status == 1
     one.close()
+
+
+def test_unused_full_space_is_let_go():
+    """One precision on the generic kernel, the other never used: the full
+    space's tables (over 100 MB here) do not stay with the handle."""
+    import torch
+    s, _, _ = _space()
+    v = np.random.default_rng(6).standard_normal((1, s.ndets))
+    s.set_sigma_route(jb.FP64, GENERIC)
+    s.sigma(v)
+    torch.cuda.synchronize()
+    free0, _ = torch.cuda.mem_get_info()
+    s.set_sigma_route(jb.FP64, FULL)
+    s.sigma(v)
+    torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] < free0 - (100 << 20)
+    s.set_sigma_route(jb.FP64, GENERIC)
+    torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] >= free0 - (16 << 20)
+    s.close()
