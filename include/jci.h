@@ -18,8 +18,11 @@
  *  - vectors are stored vector-major: v[k*ndets + i].
  *
  * Thread safety: distinct handles may be used from distinct host threads;
- * one handle must not be used concurrently.  Every call returns a status;
- * the library never exits the process.
+ * one handle must not be used concurrently.  That holds for its work on the
+ * device too: a sigma plan keeps its scratch with the handle, so sigmas of one
+ * one-group handle that are queued on several streams must be ordered by the
+ * caller (those of a truncated space are ordered by the library).  Every call
+ * returns a status; the library never exits the process.
  */
 #ifndef JCI_H
 #define JCI_H
@@ -261,7 +264,8 @@ jci_status jci_sigma_route(const jci_space *s, int precision, int *route,
 /* Fix the route with the values that jci_sigma_route reports, after
  * jci_set_integrals: 0 times both at the next sigma, 1 and 2 as above (2 with
  * mode to batch all 0 leaves the full space's plan to its autotuner).  Waits
- * for the device.  JCI_ERR_ARG for a route that the space does not have:
+ * for the device; a sigma that the caller captured before must not be replayed
+ * after it.  JCI_ERR_ARG for a route that the space does not have:
  * the full space is for spaces of at least 16384 determinants whose full
  * space has at most 16 times as many and 16384 strings of a spin, while its
  * memory fits.  No reference counterpart. */

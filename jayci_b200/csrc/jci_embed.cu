@@ -38,6 +38,7 @@ struct Embedding {
     void *v[2] = {nullptr, nullptr}, *o[2] = {nullptr, nullptr};  // full vectors, per precision
     int use[2] = {0, 0};                // per precision: 0 not timed, 1 this way, -1 the generic one
     bool none = false;                  // the space has no usable full space
+    cudaEvent_t done = nullptr;         // the last sigma through the vectors and the full scratch
 };
 
 // The pair block, row and column of full element (ia, ib) as a position in the
@@ -84,6 +85,7 @@ static void embed_drop(Embedding *e) {
 void embed_free(DeviceState *d) {
     if (!d->emb) return;
     embed_drop(d->emb);
+    if (d->emb->done) cudaEventDestroy(d->emb->done);
     delete d->emb;
     d->emb = nullptr;
 }
@@ -156,6 +158,27 @@ static bool embed_build(jci_space *s) {
     return true;
 }
 
+// Every sigma of the handle goes through the one pair of full vectors and the
+// full space's scratch, where the generic kernel has none: each waits for the
+// one before it, on whatever stream that is.  In a capture the wait and the
+// record become nodes of the graph.  The Davidson's captured iterations need
+// neither: they follow an uncaptured sigma on the same stream, and the solve
+// waits for them.
+static jci_status embed_order(const DeviceState *d, Embedding *e, cudaStream_t st, bool after) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    JCI_CUDA(cudaStreamIsCapturing(st, &cs));
+    const bool captured = cs != cudaStreamCaptureStatusNone;
+    if (captured && st == d->stream) return JCI_OK;
+    if (!e->done) JCI_CUDA(cudaEventCreateWithFlags(&e->done, cudaEventDisableTiming));
+    if (after)
+        JCI_CUDA(cudaEventRecordWithFlags(
+            e->done, st, captured ? cudaEventRecordExternal : cudaEventRecordDefault));
+    else
+        JCI_CUDA(cudaStreamWaitEvent(st, e->done,
+                                     captured ? cudaEventWaitExternal : cudaEventWaitDefault));
+    return JCI_OK;
+}
+
 template <typename T>
 static jci_status embed_run(jci_space *s, int nvec, const T *v, T *o, long long ld,
                             cudaStream_t st) {
@@ -168,16 +191,18 @@ static jci_status embed_run(jci_space *s, int nvec, const T *v, T *o, long long 
     const dim3 g((fb + 255) / 256, fa);
     T *fv = (T *)e->v[prec], *fo = (T *)e->o[prec];
     e->full->dev->sigma_skip = d->sigma_skip;
+    jci_status r = embed_order(d, e, st, false);
+    if (r) return r;
     for (int k = 0; k < nvec; k++) {
         k_embed<T, true><<<g, 256, 0, st>>>(w, e->inv[0], e->inv[1], fb, fv,
                                             const_cast<T *>(v) + k * ld);
-        jci_status r = fci_sigma(e->full, 1, fv, fo, (long long)fa * fb,
+        r = fci_sigma(e->full, 1, fv, fo, (long long)fa * fb,
                                  prec == 0 ? JCI_FP64 : JCI_FP32, st);
         if (r) return r;
         k_embed<T, false><<<g, 256, 0, st>>>(w, e->inv[0], e->inv[1], fb, fo, o + k * ld);
     }
     JCI_CUDA(cudaGetLastError());
-    return JCI_OK;
+    return embed_order(d, e, st, true);
 }
 
 jci_status embed_sigma(jci_space *s, int nvec, const void *v, void *o, long long ld, int precision,

@@ -124,3 +124,42 @@ def test_unused_full_space_is_let_go():
     torch.cuda.synchronize()
     assert torch.cuda.mem_get_info()[0] >= free0 - (16 << 20)
     s.close()
+
+
+@pytest.mark.parametrize("route", [GENERIC, FULL])
+@pytest.mark.parametrize("captured", [False, True])
+def test_two_streams_of_one_handle(route, captured):
+    """One thread queues sigmas of different vectors on two streams, as it could
+    when every truncated sigma was the scratch-free kernel; also as replays of
+    two captured graphs."""
+    import torch
+    s, _, _ = _space()
+    s.set_sigma_route(jb.FP64, route)
+    g = torch.Generator(device="cuda").manual_seed(7)
+    x = torch.randn(6, s.ndets, generator=g, dtype=torch.float64, device="cuda")
+    ref = torch.empty_like(x)
+    for k in range(6):
+        s.sigma_device(x[k].data_ptr(), ref[k].data_ptr(), 1, s.ndets, jb.FP64, 0)
+    torch.cuda.synchronize()
+    y = torch.full_like(x, float("nan"))
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+
+    def call(k, st):
+        s.sigma_device(x[k].data_ptr(), y[k].data_ptr(), 1, s.ndets, jb.FP64, st.cuda_stream)
+
+    if captured:
+        graphs = []
+        for k in range(6):
+            graphs.append(torch.cuda.CUDAGraph())
+            with torch.cuda.graph(graphs[k], stream=streams[k & 1]):
+                call(k, streams[k & 1])
+        for k in range(6):
+            with torch.cuda.stream(streams[k & 1]):
+                graphs[k].replay()
+    else:
+        for k in range(6):
+            call(k, streams[k & 1])
+    torch.cuda.synchronize()
+    assert torch.equal(y, ref)
+    s.close()
