@@ -75,12 +75,12 @@ jci_status tc_launch(const AbArgs<float> &a, int cw, int device, const float *v,
 // (jci_fci_i8.cu), FP64 and FP32.
 struct I8Tables {
     int na = 0, nb = 0, npair = 0, nchunk = 0, nrow = 0, lmax = 0;
-    unsigned long long *mx = nullptr;       // largest integral of the panel, as bits
+    unsigned long long *mx = nullptr;       // largest integral of each row and of all, as bits
     int *rowpair = nullptr;        // [128] pair of each panel row, -1: none
     uint32_t *lofs = nullptr;      // [chunk + 1] first 16-byte unit of each chunk's lists
     uint16_t *lists = nullptr;
     uint8_t *eri[2] = {nullptr, nullptr};   // digits of the integrals, per precision
-    void *rscale[2] = {nullptr, nullptr};   // scale of the integrals
+    void *rscale[2] = {nullptr, nullptr};   // scale of each row's integrals
     void *scratch[2] = {nullptr, nullptr};  // digits and scales of the vector
 };
 template <typename T>
