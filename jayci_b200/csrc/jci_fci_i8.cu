@@ -65,8 +65,9 @@
 // one instruction in seven clocks each.
 //
 // An alpha string that reaches an infinity or NaN takes its products with that
-// chunk of c in plain floating arithmetic from c itself, so such values spread
-// as they always did.
+// chunk of c in plain floating arithmetic from c itself, and with an infinity or
+// NaN among the integrals every string does, so such values spread as they always
+// did: to what H connects them to.
 #include <cuda_pipeline.h>
 
 #include <algorithm>
@@ -1095,6 +1096,7 @@ __global__ void __launch_bounds__(kIThreads, 1)
         const int m = 32 * (warp & 3) + lane;  // this lane's panel row
         const uint32_t tl = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
         const T rs = a.rscale[m];
+        const bool hfin = rs == rs;  // no infinity or NaN among the integrals
         uint32_t g = 0, r = 0, par = 0;
         bool ok = true;
         for (int is = blockIdx.x; is < nstr; is += gridDim.x) {
@@ -1159,7 +1161,7 @@ __global__ void __launch_bounds__(kIThreads, 1)
                 // this chunk's MMAs are
                 ok = ok && i8_wait(bar_full + 8 * r, par);
                 const int md = mode[r];
-                const bool bad = md == kIBad, ints = NS == 7 && md == kIOne;
+                const bool bad = md == kIBad || !hfin, ints = NS == 7 && md == kIOne && hfin;
                 ok = ok && (g < 2 || i8_wait(bar_tfree + 8 * (g & 1), ((g >> 1) - 1) & 1));
                 ok = ok && i8_wait(bar_done + 8 * acc, (g / NACC) & 1);
                 ok = __all_sync(~0u, ok);
@@ -1212,7 +1214,8 @@ __global__ void __launch_bounds__(kIThreads, 1)
                         }
                     }
                 } else if (ok) {
-                    // an infinity or NaN among the elements: the products from c itself
+                    // an infinity or NaN among the elements or the integrals: the
+                    // products from c and the integrals themselves
                     for (int idx = tid; idx < kIM * kIC; idx += 32 * kIExt) {
                         const int mm = idx / kIC, cc = idx - mm * kIC, col = c * kIC + cc;
                         const int pm = a.rowpair[mm];
