@@ -282,6 +282,12 @@ jci_status jci_sigma_set_route(jci_space *s, int precision, int route, int mode,
  * reference counterpart. */
 jci_status jci_test_expire_next_wait(jci_space *s);
 
+/* Test hook for a device with little memory left: from now on every scratch
+ * buffer of a sigma plan of more than `bytes` bytes is refused as if there were
+ * no room for it.  One-group spaces after jci_set_integrals (JCI_ERR_STATE
+ * otherwise).  No reference counterpart. */
+jci_status jci_test_limit_scratch(jci_space *s, size_t bytes);
+
 typedef struct {
         int maxiter;      /* &dalginfo defaults: 20 */
         int krymin;       /* 3 */

@@ -192,6 +192,12 @@ jci_status jci_test_expire_next_wait(jci_space *s) {
     return fci_arm_wait_expiry(s);
 }
 
+jci_status jci_test_limit_scratch(jci_space *s, size_t bytes) {
+    if (!s) return JCI_ERR_ARG;
+    if (!s->have_ints || !fci_supported(s)) return JCI_ERR_STATE;
+    return fci_limit_scratch(s, bytes);
+}
+
 void jci_davidson_defaults(jci_davidson_opts *o) {
     if (!o) return;
     memset(o, 0, sizeof(*o));

@@ -84,6 +84,7 @@ struct FciTables {
     I8Tables i8;                   // fused product on the integer tensor cores
     int i8_state = 0;              // as prs_state
     uint32_t *clist[2] = {nullptr, nullptr};  // singles of each spin for k_coulomb
+    size_t scratch_max = ~(size_t)0;  // largest scratch buffer of a plan (test hook)
     SameDense sd;                  // same-spin matrices of short string lists
     int sd_state = 0;              // as prs_state
 };
@@ -98,6 +99,22 @@ jci_status fci_arm_wait_expiry(jci_space *s) {
     if (!s->dev || !s->dev->fci) return JCI_ERR_STATE;
     s->dev->fci->wave_expire = 1;
     return JCI_OK;
+}
+
+jci_status fci_limit_scratch(jci_space *s, size_t bytes) {
+    if (!s->dev || !s->dev->fci) return JCI_ERR_STATE;
+    s->dev->fci->scratch_max = bytes;
+    return JCI_OK;
+}
+
+// A plan's scratch buffer; JCI_ERR_NOMEM, with no error left behind, when there
+// is no room.
+template <typename P>
+static jci_status scratch_alloc(const FciTables *f, P **p, size_t bytes) {
+    if (bytes <= f->scratch_max && cudaMalloc((void **)p, bytes) == cudaSuccess) return JCI_OK;
+    cudaGetLastError();
+    *p = nullptr;
+    return JCI_ERR_NOMEM;
 }
 
 jci_status fci_wait_status(jci_space *s) {
@@ -1580,7 +1597,9 @@ static jci_status launch_mixed_blk_t(jci_space *s, const MixBArgs<T> &ab, const 
         JCI_CUDA(cudaStreamIsCapturing(st, &cs));
         if (cs != cudaStreamCaptureStatusNone) return JCI_ERR_STATE;
         const int g = std::max(1, std::min(ab.m.na, nsm * occ));
-        JCI_CUDA(cudaMalloc(&f->tbufk[prec], (size_t)g * ab.m.mrows * kMixBlock * sizeof(T)));
+        jci_status r = scratch_alloc(f, &f->tbufk[prec],
+                                     (size_t)g * ab.m.mrows * kMixBlock * sizeof(T));
+        if (r) return r;
         f->mixk_grid[prec] = g;
     }
     int grid = f->mixk_grid[prec];
@@ -1674,7 +1693,9 @@ static jci_status launch_wave(jci_space *s, const MixArgs<T> &m, const T *v, T *
     int grid = nsm * (per_sm > 0 && per_sm < occ ? per_sm : occ);
     if ((long long)m.na * (ngi + nhi) + grid >= (1ll << 31)) return JCI_ERR_SPACE;
     if (!f->wbuf[prec]) {
-        JCI_CUDA(cudaMalloc(&f->wbuf[prec], (size_t)kWaveBufs * m.mrows * m.nbp * sizeof(T)));
+        jci_status r = scratch_alloc(f, &f->wbuf[prec],
+                                     (size_t)kWaveBufs * m.mrows * m.nbp * sizeof(T));
+        if (r) return r;
         JCI_CUDA(cudaMalloc(&f->wctl[prec], sizeof(WaveCtl)));
     }
     JCI_CUDA(cudaMemsetAsync(f->wctl[prec], 0, sizeof(WaveCtl), st));
@@ -1820,7 +1841,8 @@ static jci_status launch_mixed(jci_space *s, const FciArgs<T> &fa, const T *v, T
         JCI_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, d->device));
         int grid = std::max(1, std::min(m.na, nsm * std::max(occ, 1)));
         size_t bytes = (size_t)grid * m.mrows * m.nbp * sizeof(T);
-        JCI_CUDA(cudaMalloc(&f->tbuf[prec], bytes));
+        jci_status r = scratch_alloc(f, &f->tbuf[prec], bytes);
+        if (r) return r;
         f->mix_grid[prec] = grid;
         f->mix_occ[prec] = std::max(occ, 1);
         f->nsm = nsm;
@@ -1959,7 +1981,7 @@ static jci_status launch_ab(jci_space *s, const FciArgs<T> &fa, const T *v, T *o
     if (tx == kI8Engine) {
         FciTables *f = s->dev->fci;
         jci_status r = i8_tables(s, st);
-        if (!r) r = i8_scratch(&f->i8, sizeof(T));
+        if (!r) r = i8_scratch(&f->i8, sizeof(T), f->scratch_max);
         if (r) return r;
         if (singles) {
             StreamArgs<T> al;
@@ -2081,7 +2103,7 @@ static jci_status launch_hs(jci_space *s, const StreamArgs<T> &be, const T *ct, 
         s->dev->sigma_gen++;
         f->hbuf[prec] = nullptr;
         f->hbytes[prec] = 0;
-        JCI_CUDA(cudaMalloc(&f->hbuf[prec], need));
+        if ((r = scratch_alloc(f, &f->hbuf[prec], need))) return r;
         f->hbytes[prec] = need;
     }
     return hs_launch<T>(f->hst, f->na, f->npair, be.jc, ct, tau, be.skip, (T *)f->hbuf[prec],
@@ -2109,7 +2131,8 @@ static jci_status pair_scratch(jci_space *s, int items, cudaStream_t st, T **E) 
         s->dev->sigma_gen++;
         f->pbuf[prec] = nullptr;
         f->pbytes[prec] = 0;
-        JCI_CUDA(cudaMalloc(&f->pbuf[prec], need));
+        jci_status r = scratch_alloc(f, &f->pbuf[prec], need);
+        if (r) return r;
         f->pbytes[prec] = need;
     }
     *E = (T *)f->pbuf[prec];
@@ -2157,7 +2180,10 @@ template <typename T>
 static jci_status stream_scratch(FciTables *f, T **ct, T **tau) {
     const int prec = sizeof(T) == 8 ? 0 : 1;
     size_t n = (size_t)f->na * f->nb;
-    if (!f->sbuf[prec]) JCI_CUDA(cudaMalloc(&f->sbuf[prec], 2 * n * sizeof(T)));
+    if (!f->sbuf[prec]) {
+        jci_status r = scratch_alloc(f, &f->sbuf[prec], 2 * n * sizeof(T));
+        if (r) return r;
+    }
     *ct = (T *)f->sbuf[prec];
     *tau = *ct + n;
     return JCI_OK;
@@ -2366,20 +2392,36 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
     size_t w = sizeof(T);
     long long n = (long long)f->na * f->nb;
     T *v = nullptr, *o = nullptr;
-    JCI_CUDA(cudaMalloc(&v, n * w));
-    JCI_CUDA(cudaMalloc(&o, n * w));
+    if (cudaMalloc(&v, n * w) != cudaSuccess || cudaMalloc(&o, n * w) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(v);
+        return JCI_ERR_NOMEM;
+    }
     JCI_CUDA(cudaMemsetAsync(v, 0, n * w, st));
     const int nts[] = {128, 256, 512, 1024};
     const int Rs[] = {1, 2, 4, 8, 16};
     cudaEvent_t e0, e1;
     JCI_CUDA(cudaEventCreate(&e0));
     JCI_CUDA(cudaEventCreate(&e1));
-    jci_status err = JCI_OK;
+    // A candidate that cannot run -- no room for its scratch or its tables, a
+    // space outside its limits -- is dropped; the last such error is returned
+    // when none can.
+    jci_status err = JCI_OK, last = JCI_ERR_SPACE;
+    auto drop = [&]() {
+        if (err) {
+            last = err;
+            cudaGetLastError();
+        }
+        err = JCI_OK;
+    };
     // ms per call of fn: one untimed call, then two timed -- or one, when a
     // call takes more than 50 ms (large spaces: launch noise is then far
     // below the differences between candidates, and tuning time matters)
     auto timeit = [&](auto fn) -> float {
-        if (err || (err = fn())) return 1e30f;
+        if ((err = fn())) {
+            drop();
+            return 1e30f;
+        }
         float ms = 0.f;
         int reps = 0;
         for (int k = 0; k < 2 && !err; k++) {
@@ -2393,7 +2435,9 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
             reps++;
             if (t > 50.f) break;
         }
-        return err ? 1e30f : ms / reps;
+        if (!err) return ms / reps;
+        drop();
+        return 1e30f;
     };
     auto useful = [&](int nt) {
         int items = (f->nb + nt - 1) / nt;
@@ -2419,8 +2463,13 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
                 best_of([&] { return run_plan<T>(s, a, 7, kSplitSingles, kI8Engine, B, v, o, st); });
             if (ms < bests) { bests = ms; bsB = B; }
         }
-        if (err) cudaGetLastError();
-        err = JCI_OK;  // a space too large for its scratch just drops the plan
+        if (bests >= 1e30f) {  // what it did get is room for the other plans
+            cudaFree(f->sbuf[prec]);
+            cudaFree(f->pbuf[prec]);
+            cudaFree(f->i8.scratch[prec]);
+            f->sbuf[prec] = f->pbuf[prec] = f->i8.scratch[prec] = nullptr;
+            f->pbytes[prec] = 0;
+        }
     }
     // From 2^21 determinants on it beats every other plan (FP64, against the
     // best of the others: 1.60 to 1.85 ms at 2.9 M determinants, 6.8 to 12.4 at
@@ -2492,9 +2541,10 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
     // modes 3, 4: streaming passes on C and C^T, the transposes, the product
     float best3 = 1e30f;
     int b3a = 0, b3b = 0;
-    if (bsprod < 1e30f) {
-        T *ct = nullptr, *tau = nullptr;
-        if (!err) err = stream_scratch<T>(f, &ct, &tau);
+    T *ct = nullptr, *tau = nullptr;
+    const bool streamed = bsprod < 1e30f && !(err = stream_scratch<T>(f, &ct, &tau));
+    drop();
+    if (streamed) {
         StreamArgs<T> al, be;
         stream_args(a, al, be);
         float ba = 1e30f, bb = 1e30f;
@@ -2518,9 +2568,7 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
     float best6 = 1e30f;
     int b6s = 0, b6i = 1;
     bool pairs = false;  // the hole-string variants (5, 6) can run
-    if (bsprod < 1e30f && group_possible(f) && !err) {
-        T *ct = nullptr, *tau = nullptr;
-        err = stream_scratch<T>(f, &ct, &tau);
+    if (streamed && group_possible(f)) {
         StreamArgs<T> al, be;
         stream_args(a, al, be);
         be.nd = 0;
@@ -2550,7 +2598,6 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
             return q ? q : launch_transposes<T>(f, v, ct, o, tau, true, nullptr, st);
         });
         if (found && gg < 1e30f) best6 = bs + gg + tt + bsprod;
-        err = JCI_OK;  // a space the group tables cannot hold just drops the plan
     }
     // mode 5 with the same-spin part as dense products, end to end.  Measured
     // (us, best of the other plans -> this one): N electrons in N orbitals
@@ -2587,10 +2634,9 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
     cudaEventDestroy(e1);
     cudaFree(v);
     cudaFree(o);
-    if (err) return err;
-    if (!b0nt && !b1nt && !(b3a && b3b) && best6 >= 1e30f && bests >= 1e30f &&
+    if (best0 >= 1e30f && best1 >= 1e30f && best3 >= 1e30f && best6 >= 1e30f && bests >= 1e30f &&
         bestd >= 1e30f)
-        return JCI_ERR_SPACE;
+        return last;
     int mode = 0;
     float best = best0;
     if (b1nt && best1 < best) { mode = b1mode; best = best1; }
@@ -2635,6 +2681,11 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
     if (eng != kI8Engine && f->i8.scratch[prec]) {  // the integer engine's digits are not needed
         cudaFree(f->i8.scratch[prec]);
         f->i8.scratch[prec] = nullptr;
+    }
+    if (!(groups && f->tuned_B[prec] >= 5) && f->pbuf[prec]) {  // nor the hole strings' E blocks
+        cudaFree(f->pbuf[prec]);
+        f->pbuf[prec] = nullptr;
+        f->pbytes[prec] = 0;
     }
     if (mode != 1 && mode != 3 && mode != 6 && f->tbuf[prec]) {  // the product panels are not needed
         cudaFree(f->tbuf[prec]);
@@ -2761,7 +2812,7 @@ static jci_status force_plan(jci_space *s, int precision, int mode, int nt, int 
     }
     if (mode == 4 || mode == 5 || mode == 7) {  // tables are built here, outside any capture
         AbTables *t = nullptr;
-        jci_status r = R == kI8Engine ? i8_scratch(&f->i8, w)
+        jci_status r = R == kI8Engine ? i8_scratch(&f->i8, w, f->scratch_max)
                                       : ab_tables(s, ab_table_tx(R), s->dev->stream, &t);
         if (r) return r;
     }

@@ -1432,11 +1432,14 @@ static I8Scratch i8_scratch_layout(const I8Tables &t, size_t w, int ns) {
     return l;
 }
 
-jci_status i8_scratch(I8Tables *t, size_t w) {
+jci_status i8_scratch(I8Tables *t, size_t w, size_t most) {
     const int p = w == 8 ? 0 : 1, ns = p ? kDigits<float> : kDigits<double>;
     if (t->scratch[p]) return JCI_OK;
-    JCI_CUDA(cudaMalloc(&t->scratch[p], i8_scratch_layout(*t, w, ns).total));
-    return JCI_OK;
+    const size_t bytes = i8_scratch_layout(*t, w, ns).total;
+    if (bytes <= most && cudaMalloc(&t->scratch[p], bytes) == cudaSuccess) return JCI_OK;
+    cudaGetLastError();
+    t->scratch[p] = nullptr;
+    return JCI_ERR_NOMEM;
 }
 
 // o += the alpha-single x beta-single part of H v.

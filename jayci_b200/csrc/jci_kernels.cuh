@@ -17,6 +17,8 @@ jci_status fci_wait_status(jci_space *s);
 // Test hook: the next launch of the shared-panel product leaves the GEMM
 // items of its first rows undone, so that its gathers' waits expire.
 jci_status fci_arm_wait_expiry(jci_space *s);
+// Test hook: scratch buffers of more than this many bytes are refused.
+jci_status fci_limit_scratch(jci_space *s, size_t bytes);
 jci_status fci_prepare(jci_space *s);
 jci_status fci_sigma(jci_space *s, int nvec, const void *v, void *sig, long long ld,
                      int precision, cudaStream_t st);
@@ -95,7 +97,7 @@ jci_status i8_tables_build(const jci_space *s, int npair, I8Tables *t);
 void i8_tables_free(I8Tables *t);
 jci_status i8_fill(I8Tables *t, const double *m2, cudaStream_t st);
 size_t i8_smem(const I8Tables &t, int sa, size_t w);
-jci_status i8_scratch(I8Tables *t, size_t w);
+jci_status i8_scratch(I8Tables *t, size_t w, size_t most);
 template <typename T>
 jci_status i8_launch(const I8Tables &t, const I8Input<T> &in, int device, const T *v, T *o,
                      int *status, cudaStream_t st);
