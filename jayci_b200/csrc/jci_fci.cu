@@ -2379,6 +2379,25 @@ static jci_status run_plan(jci_space *s, FciArgs<T> a, int mode, int nt, int R, 
     return launch_mixed<T>(s, a, v, o, st, R);
 }
 
+// The vector that plans are timed on: pseudo-random elements that shrink by
+// 10^0.4 for every electron above the lowest orbitals, over some six decades
+// at FCI(16,16).  The digit product's time depends on how its vector is graded
+// (FCI(14,14) FP64 7.2 ms a sigma for a random one, 8.8 for a CI vector); a
+// solve's vectors look like this one.
+template <typename T>
+__global__ void k_tune_vector(int na, int nb, int nela, int nelb,
+                              const uint64_t *__restrict__ oa, const uint64_t *__restrict__ ob,
+                              T *__restrict__ v) {
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i >= (long long)na * nb) return;
+    const int lev = __popcll(oa[i / nb] >> nela) + __popcll(ob[i % nb] >> nelb);
+    uint32_t x = (uint32_t)i * 2654435761u + (uint32_t)(i >> 32);
+    x = (x ^ (x >> 16)) * 2246822519u;
+    x ^= x >> 13;
+    const float u = (float)(int32_t)x * (1.f / 2147483648.f);
+    v[i] = (T)(u * exp10f(-0.4f * lev));
+}
+
 // Pick the plan for this space by timing the admissible candidates on
 // scratch vectors (modes as in run_plan).  The row kernel, the stream passes
 // and the product kernels are tuned one by one; the best configuration of
@@ -2397,7 +2416,8 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
         cudaFree(v);
         return JCI_ERR_NOMEM;
     }
-    JCI_CUDA(cudaMemsetAsync(v, 0, n * w, st));
+    k_tune_vector<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
+        f->na, f->nb, d->t[0].nelec, d->t[1].nelec, d->t[0].occ, d->t[1].occ, v);
     const int nts[] = {128, 256, 512, 1024};
     const int Rs[] = {1, 2, 4, 8, 16};
     cudaEvent_t e0, e1;
@@ -2471,10 +2491,14 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
             f->pbytes[prec] = 0;
         }
     }
-    // From 2^21 determinants on it beats every other plan (FP64, against the
-    // best of the others: 1.60 to 1.85 ms at 2.9 M determinants, 6.8 to 12.4 at
-    // 11.8 M, 123 to 232 at 165.6 M; below, at 0.85 M, they lie within a few
-    // percent), and timing those would take half a minute at the largest.
+    // From 2^21 determinants on no other plan beats it, and timing those would
+    // take half a minute at the largest.  Measured on the graded vector (ms,
+    // split / best of the others; electrons in orbitals, alpha singles): 13 in 13
+    // (42) FP64 2.21 / 2.21, FP32 1.23 / 1.45; 10 in 14 (45) 3.10 / 3.27, 1.67 /
+    // 1.95; 9 in 15 (50) 3.34 / 3.66, 1.90 / 2.25; 12 in 14 (48) 7.09 / 7.92,
+    // 4.06 / 4.76; 14 in 14 (49) 9.31 / 10.8, 4.98 / 5.96; 10 in 16 (55) 15.0 /
+    // 18.0, 7.80 / 9.74; below, 12 in 12 0.71 / 0.49, 0.45 / 0.41, 8 in 15 (1.9
+    // million) 1.37 / 1.51, 0.86 / 0.98.
     const bool only_split = bests < 1e30f && n >= (1ll << 21);
     // mode 0: one kernel, R staged rows
     float best0 = 1e30f;
