@@ -264,7 +264,7 @@ jci_status jci_sigma_route(const jci_space *s, int precision, int *route,
 /* Fix the route with the values that jci_sigma_route reports, after
  * jci_set_integrals: 0 times both at the next sigma, 1 and 2 as above (2 with
  * mode to batch all 0 leaves the full space's plan to its autotuner).  Waits
- * for the device; a sigma that the caller captured before must not be replayed
+ * for the sigmas that are queued; a sigma that the caller captured before must not be replayed
  * after it.  JCI_ERR_ARG for a route that the space does not have:
  * the full space is for spaces of at least 16384 determinants whose full
  * space has at most 16 times as many and 16384 strings of a spin, while its
@@ -381,7 +381,17 @@ typedef struct {
  * at once (0 = 80 % of free device memory); slots = solves in flight. */
 jci_status jci_server_create(size_t hbm_budget_bytes, int slots,
                              jci_server **out);
-/* Queue a request; returns JCI_ERR_BUSY if its estimated footprint exceeds
+/* Device memory that a request is admitted with under a budget of this many
+ * bytes (0: none): the Davidson panels, the tables, the scratch of the sigma
+ * plans it may tune and, for a truncated space, the full CI space that sigma
+ * may run through.  *generic = 1 where that space does not fit, so that the
+ * server keeps sigma to the generic kernel (jci_sigma_set_route); a request
+ * whose plans do not fit either is admitted with the whole budget, alone.
+ * JCI_ERR_BUSY where the panels and tables alone exceed the budget.  Needs no
+ * device. */
+jci_status jci_request_footprint(const jci_request *req, size_t budget,
+                                 size_t *bytes, int *generic);
+/* Queue a request; returns JCI_ERR_BUSY if its panels and tables exceed
  * the whole budget, JCI_ERR_SPACE / JCI_ERR_ARG for invalid requests. */
 jci_status jci_server_submit(jci_server *srv, const jci_request *req,
                              long long *ticket);

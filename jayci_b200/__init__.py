@@ -306,6 +306,20 @@ class Result(ctypes.Structure):
                 ("sigma_seconds", ctypes.c_double)]
 
 
+def request_footprint(general, nroots=1, krymin=None, krymax=24, precision=FP64, budget_bytes=0):
+    """(bytes, generic) that a server of this budget admits such a solve with
+    (jci_request_footprint; no device needed)."""
+    r = Request(*general, None, None, 0.0, 0.0, nroots, krymin or max(nroots, 4), krymax, 1, 8,
+                1e-8, precision, 1e-4, 1, -1)
+    f = lib().jci_request_footprint
+    f.argtypes = [ctypes.POINTER(Request), ctypes.c_size_t, ctypes.POINTER(ctypes.c_size_t),
+                  ctypes.POINTER(ctypes.c_int)]
+    n, g = ctypes.c_size_t(), ctypes.c_int()
+    _check(f(ctypes.byref(r), budget_bytes, ctypes.byref(n), ctypes.byref(g)),
+           "request_footprint")
+    return n.value, bool(g.value)
+
+
 class Server:
     """Continuous-batching CI solve server (jci_server_*): `slots` solves in
     flight, admitted by estimated HBM footprint within `budget_bytes`."""

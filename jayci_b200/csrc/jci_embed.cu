@@ -113,6 +113,15 @@ jci_status embed_set_integrals(jci_space *s) {
     return e && e->full ? embed_integrals(s) : JCI_OK;
 }
 
+bool embed_strings(const jci_space *s, long long n[2]) {
+    const int na = s->ci_aelec, nb = s->ci_belec, no = s->ci_orbs;
+    if (s->ndets < kEmbedMin || no > 64 || na - nb < 0 || na - nb > 1) return false;
+    n[0] = binom(no, na);
+    n[1] = binom(no, nb);
+    return n[0] >= 1 && n[1] >= 1 && n[0] <= kEmbedStrings && n[1] <= kEmbedStrings &&
+           n[0] * n[1] <= kEmbedRatio * s->ndets;
+}
+
 // The full space and the string maps; false when there is none within the
 // limits or the device's free memory.
 static bool embed_build(jci_space *s) {
@@ -120,11 +129,9 @@ static bool embed_build(jci_space *s) {
     Embedding *e = d->emb;
     if (e->full) return true;
     const int na = s->ci_aelec, nb = s->ci_belec, no = s->ci_orbs;
-    if (s->ndets < kEmbedMin || no > 64 || na - nb < 0 || na - nb > 1) return false;
-    const long long fa = binom(no, na), fb = binom(no, nb);
-    if (fa < 1 || fb < 1 || fa > kEmbedStrings || fb > kEmbedStrings ||
-        fa * fb > kEmbedRatio * s->ndets)
-        return false;
+    long long n[2];
+    if (!embed_strings(s, n)) return false;
+    const long long fa = n[0], fb = n[1];
     // vectors, transposes and digits of both precisions, and room to spare
     size_t mfree = 0, mtotal = 0;
     if (cudaMemGetInfo(&mfree, &mtotal) != cudaSuccess ||
@@ -308,7 +315,9 @@ jci_status embed_set_route(jci_space *s, int precision, int route, int mode, int
     if (!d->emb) d->emb = new (std::nothrow) Embedding();
     Embedding *e = d->emb;
     if (!e) return JCI_ERR_NOMEM;
-    JCI_CUDA(cudaDeviceSynchronize());  // nothing that is let go of is still in use
+    // nothing that is let go of is still in use
+    JCI_CUDA(cudaStreamSynchronize(d->stream));
+    if (e->done) JCI_CUDA(cudaEventSynchronize(e->done));
     if (route == kRouteFull) {
         if (!embed_build(s)) return JCI_ERR_ARG;
         jci_status r = embed_vectors(e, prec) ? JCI_OK : JCI_ERR_NOMEM;

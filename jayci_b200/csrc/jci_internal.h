@@ -77,6 +77,10 @@ jci_status davidson(jci_space *s, const jci_davidson_opts *o,
                     double *energies, double *civec, jci_davidson_stats *st);
 jci_status davidson_vectors(jci_space *s, int k, double *out);
 
+// Strings of each spin of the full CI space that sigma of this truncated space
+// may run through (jci_embed.cu); false when its size rules that out.
+bool embed_strings(const jci_space *s, long long n[2]);
+
 // I/O helpers (jci_io.cpp).
 jci_status write_vectors(const char *path, int dim, int len, const double *v);
 

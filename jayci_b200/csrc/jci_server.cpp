@@ -9,7 +9,8 @@
 // overlap on the device.  Spaces are cached by their &general values
 // (device tables, tuned sigma plans and Davidson buffers are reused by the
 // next request on the same space: a geometry scan re-uploads integrals
-// only), and a request may start from the Ritz vectors of an earlier one:
+// only); idle ones are given up, the least recently used first, when they and
+// the running solves outgrow the budget.  A request may start from the Ritz vectors of an earlier one:
 // it is not started before that one has finished, so the steps of a scan
 // run in order while other scans fill the remaining slots.
 //
@@ -41,17 +42,15 @@ using Clock = std::chrono::steady_clock;
 
 namespace {
 
-using Key = std::tuple<int, int, int, int, int, int, int>;
-
-Key key_of(const jci_request &r) {
-    return Key{r.electrons, r.orbitals, r.nfrozen, r.ndocc, r.nactive, r.nfrzvirt, r.xlevel};
-}
+// &general values, and whether sigma is kept to the generic kernel
+using Key = std::tuple<int, int, int, int, int, int, int, bool>;
 
 struct Job {
     long long id = 0;
     jci_request req{};
     std::vector<double> m1, m2;
     size_t footprint = 0;
+    bool generic = false;         // no room for the full CI space in the budget
     long long ndets = 0;
     jci_space *fresh = nullptr;   // host-built space, used if no cached one
     bool done = false;
@@ -61,9 +60,52 @@ struct Job {
     Clock::time_point t_submit, t_start, t_end;
 };
 
-// Device footprint of one solve: Davidson panels, device tables, sigma
-// plan scratch (generous: every panel the product kernel may allocate).
-size_t estimate_footprint(const jci_space *s, const jci_request &r) {
+Key key_of(const Job &j) {
+    const jci_request &r = j.req;
+    return Key{r.electrons, r.orbitals, r.nfrozen, r.ndocc, r.nactive, r.nfrzvirt, r.xlevel,
+               j.generic};
+}
+
+struct Footprint {
+    size_t core = 0;   // what every solve of the space needs
+    size_t plans = 0;  // scratch and tables of the sigma plans that it may tune
+    size_t full = 0;   // the full CI space behind a truncated one, 0: not used
+};
+
+// Scratch and tables of the one-group sigma plans, n orbitals, ns[spin] strings
+// of ne[spin] electrons.  Plans that find no room are dropped by the autotuner.
+size_t plan_bytes(const long long ns[2], const int ne[2], int n, bool mixed) {
+    const long long N = ns[0] * ns[1], npair = (long long)n * (n + 1) / 2;
+    size_t b = 0;
+    for (int w : {8, 4}) {
+        if (w == 4 && !mixed) continue;
+        const long long nchunk = (ns[1] + 47) / 48;
+        // 8-bit digits of the vector, masks, flags, scales (jci_fci_i8.cu)
+        b += (w == 8 ? 7ull : 4ull) * 48 * nchunk * ns[0] + 17ull * nchunk * ns[0] +
+             nchunk * 48ull * w + 12ull * (ns[0] + ns[1]);
+        if (w == 4) b += 16ull * N;  // autotune and streaming scratch of FP32
+        // E blocks of the hole-string doubles and singles (jci_fci_pairs.cu)
+        size_t e = 0;
+        for (int sp = 0; sp < 2; sp++) {
+            const size_t col = (size_t)ns[sp] * (ne[sp] * (ne[sp] - 1) / 2) * w;
+            e = std::max(e, std::min<size_t>(4ull << 30, col * ns[sp ^ 1]) + 64 * col);
+        }
+        const size_t hcol = (size_t)ns[1] * ne[1] * w;
+        b += e + std::min<size_t>(1ull << 30, hcol * ns[0]) + 64 * hcol;
+    }
+    for (int sp = 0; sp < 2; sp++) {
+        const long long k = ne[sp], sing = k * (n - k);
+        b += 10ull * ns[sp] * (k * (k - 1) / 2);           // hole-string tables
+        b += 4ull * ns[sp] * sing + 24ull * ns[sp] * k;    // Coulomb lists, singles' hole strings
+        b += 12ull * ns[sp] * sing;                        // chunk lists of the products
+        if (ns[sp] <= 2048) b += 12ull * ns[sp] * ((ns[sp] + 31) / 32 * 32);  // same-spin matrices
+    }
+    return b + 2ull * npair * 128 * 12;                    // digits of the integrals
+}
+
+// Device memory of one solve: Davidson panels, device tables, sigma plan
+// scratch (generous: every panel the product kernel may allocate).
+Footprint estimate_footprint(const jci_space *s, const jci_request &r) {
     long long n = s->ndets, ld = (n + 31) / 32 * 32;
     size_t b = 8ull * ld * (3ull * r.krymax + 2);
     if (r.precision == JCI_MIXED) b += 8ull * ld * std::max(r.krymin, r.nroots);
@@ -82,7 +124,42 @@ size_t estimate_footprint(const jci_space *s, const jci_request &r) {
         b += 12ull * grid * (npair + 1) * nbp;
     }
     b += 16ull * (npair * (npair + 1) / 2 + npair);  // integrals FP64 + FP32
-    return b + (64ull << 20);                         // runtime slack
+    Footprint f;
+    f.core = b + (64ull << 20);                       // runtime slack
+    const bool mixed = r.precision == JCI_MIXED;
+    const int ne[2] = {s->ci_aelec, s->ci_belec};
+    if (n <= 2048) f.plans += 12ull * n * ((n + 31) / 32 * 32);  // H itself
+    if (s->sp[0].ngrp == 1 && s->sp[1].ngrp == 1) {
+        const long long ns[2] = {s->sp[0].nstr, s->sp[1].nstr};
+        f.plans += plan_bytes(ns, ne, s->ci_orbs, mixed);
+    } else {
+        long long ns[2];
+        if (embed_strings(s, ns)) {
+            const long long N = ns[0] * ns[1];
+            // its vectors, transposes, autotune vectors and diagonal; its tables
+            f.full = plan_bytes(ns, ne, s->ci_orbs, mixed) + (mixed ? 72ull : 60ull) * N;
+            for (int sp = 0; sp < 2; sp++) {
+                const long long k = ne[sp], h = s->ci_orbs - k;
+                f.full += ns[sp] * (40ull * k * h + 24ull * (k * (k - 1) / 2) * (h * (h - 1) / 2) +
+                                    12ull * npair + 64);
+            }
+            // panels of the plans that smaller full spaces time
+            if (N < (1ll << 21))
+                f.full += 12ull * std::min<long long>(ns[0], 148 * 4) * (npair + 1) *
+                          ((ns[1] + 63) / 64 * 64);
+            f.full += 64ull << 20;
+        }
+    }
+    return f;
+}
+
+// What a request is admitted with under a budget: everything that it may
+// allocate; without the full CI space where that does not fit (the generic
+// kernel needs none), and the whole budget, so that it runs alone, where the
+// plans' scratch does not either (the autotuner drops what finds no room).
+size_t admitted_bytes(const Footprint &f, size_t budget, bool *generic) {
+    *generic = f.full && f.core + f.plans + f.full > budget;
+    return std::min(budget, f.core + f.plans + (*generic ? 0 : f.full));
 }
 
 }  // namespace
@@ -100,22 +177,35 @@ struct jci_server {
     std::vector<std::thread> workers;
     // idle spaces by key (least recently used first); spaces in use are
     // owned by the worker running them
-    std::list<std::pair<Key, jci_space *>> idle;
+    struct Idle {
+        Key key;
+        jci_space *space;
+        size_t bytes;   // what it may hold
+    };
+    std::list<Idle> idle;
     size_t idle_max = 8;
 };
 
 static void run_job(jci_server *srv, Job *job) {
     const jci_request &r = job->req;
-    Key k = key_of(r);
+    Key k = key_of(*job);
     jci_space *s = nullptr;
     {
         std::lock_guard<std::mutex> g(srv->mu);
         for (auto it = srv->idle.begin(); it != srv->idle.end(); ++it)
-            if (it->first == k) {
-                s = it->second;
+            if (it->key == k) {
+                s = it->space;
                 srv->idle.erase(it);
                 break;
             }
+        // idle spaces make room, the least recently used first
+        size_t held = 0;
+        for (auto &x : srv->idle) held += x.bytes;
+        while (!srv->idle.empty() && srv->used + held > srv->budget) {
+            held -= srv->idle.front().bytes;
+            jci_space_destroy(srv->idle.front().space);
+            srv->idle.pop_front();
+        }
     }
     if (s) {
         jci_space_destroy(job->fresh);
@@ -125,6 +215,8 @@ static void run_job(jci_server *srv, Job *job) {
     job->fresh = nullptr;
     jci_status st = jci_set_integrals(s, job->m1.data(), job->m2.data(), s->ci_orbs, r.nucrep,
                                       r.frzcore);
+    for (int p : {JCI_FP64, JCI_FP32})
+        if (!st && job->generic) st = jci_sigma_set_route(s, p, 1, 0, 0, 0, 0);
     std::vector<double> init;
     int warm = 0;
     if (!st && r.warm_from > 0) {
@@ -188,9 +280,9 @@ static void run_job(jci_server *srv, Job *job) {
     if (st == JCI_ERR_CUDA || st == JCI_ERR_NODEVICE) {
         jci_space_destroy(s);
     } else {
-        srv->idle.emplace_back(k, s);
+        srv->idle.push_back({k, s, job->footprint});
         while (srv->idle.size() > srv->idle_max) {
-            jci_space_destroy(srv->idle.front().second);
+            jci_space_destroy(srv->idle.front().space);
             srv->idle.pop_front();
         }
     }
@@ -258,6 +350,21 @@ jci_status jci_server_create(size_t budget, int slots, jci_server **out) {
     return JCI_OK;
 }
 
+jci_status jci_request_footprint(const jci_request *req, size_t budget, size_t *bytes,
+                                 int *generic) {
+    if (!req || !bytes || !generic) return JCI_ERR_ARG;
+    jci_space *s = nullptr;
+    jci_status st = jci_space_create(req->electrons, req->orbitals, req->nfrozen, req->ndocc,
+                                     req->nactive, req->nfrzvirt, req->xlevel, &s);
+    if (st) return st;
+    bool g = false;
+    const Footprint f = estimate_footprint(s, *req);
+    *bytes = admitted_bytes(f, budget ? budget : ~(size_t)0, &g);
+    *generic = g;
+    jci_space_destroy(s);
+    return budget && f.core > budget ? JCI_ERR_BUSY : JCI_OK;
+}
+
 jci_status jci_server_submit(jci_server *srv, const jci_request *req, long long *ticket) {
     if (!srv || !req || !ticket || !req->moints1 || !req->moints2) return JCI_ERR_ARG;
     if (req->nroots < 1 || req->nroots > JCI_MAX_ROOTS || req->krymin < req->nroots ||
@@ -280,9 +387,10 @@ jci_status jci_server_submit(jci_server *srv, const jci_request *req, long long 
     job->m2.assign(req->moints2, req->moints2 + n2);
     job->req.moints1 = job->req.moints2 = nullptr;
     job->ndets = s->ndets;
-    job->footprint = estimate_footprint(s, *req);
+    const Footprint need = estimate_footprint(s, *req);
+    job->footprint = admitted_bytes(need, srv->budget, &job->generic);
     std::lock_guard<std::mutex> g(srv->mu);
-    if (job->footprint > srv->budget) {
+    if (need.core > srv->budget) {
         jci_space_destroy(s);
         return JCI_ERR_BUSY;
     }
@@ -346,7 +454,7 @@ void jci_server_destroy(jci_server *srv) {
     }
     srv->cv_work.notify_all();
     for (auto &t : srv->workers) t.join();
-    for (auto &p : srv->idle) jci_space_destroy(p.second);
+    for (auto &p : srv->idle) jci_space_destroy(p.space);
     for (auto &j : srv->jobs) jci_space_destroy(j.second->fresh);
     delete srv;
 }
