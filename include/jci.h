@@ -164,7 +164,11 @@ jci_status jci_sigma(jci_space *s, int nvec, const double *v, double *sigma,
  * elements); element type double for JCI_FP64, float for JCI_FP32.  The
  * work is queued on `stream` (a cudaStream_t).  NULL = the handle's own
  * stream, ordered after the work already queued on the legacy default
- * stream, which in turn waits for the sigma before its later work. */
+ * stream, which in turn waits for the sigma before its later work.  Every wait
+ * inside a sigma kernel is bounded; one that runs out leaves that sigma
+ * incomplete, and the next call on the handle that finds it out (this one,
+ * without waiting for the device, jci_sigma or jci_davidson) returns
+ * JCI_ERR_TIMEOUT and does nothing else. */
 jci_status jci_sigma_device(jci_space *s, int nvec, const void *v,
                             void *sigma, long long ld, int precision,
                             void *stream);
@@ -274,10 +278,11 @@ jci_status jci_sigma_set_route(jci_space *s, int precision, int route, int mode,
 
 /* Test hook for the device-side wait bounds.  The next sigma whose product
  * runs through the row panels shared by all CTAs (plan rows >= 32) leaves
- * the panel work of its first two alpha rows undone, so the gathers that
+ * the panel work of its first two alpha rows undone, and one through the digit
+ * product (plan rows 128) the first chunk of its first CTA, so the gathers that
  * depend on it wait until their bound (about one second) expires; that
- * sigma's output is then incomplete and the next host-synchronising call
- * (jci_sigma, jci_davidson) returns JCI_ERR_TIMEOUT, after which the space
+ * sigma's output is then incomplete and that call (jci_sigma, jci_davidson) or
+ * the next jci_sigma_device returns JCI_ERR_TIMEOUT, after which the space
  * works as before.  JCI_ERR_STATE for a space without device tables.  No
  * reference counterpart. */
 jci_status jci_test_expire_next_wait(jci_space *s);

@@ -83,6 +83,8 @@ jci_status jci_sigma_device(jci_space *s, int nvec, const void *v, void *sig, lo
                             int precision, void *stream) {
     if (!s) return JCI_ERR_ARG;
     if (precision != JCI_FP64 && precision != JCI_FP32) return JCI_ERR_ARG;
+    // an earlier call's wait that has expired meanwhile (a host read)
+    if (jci_status r = fci_wait_status(s)) return r;
     if (stream || !s->dev) return device_sigma(s, nvec, v, sig, ld, precision, stream);
     // NULL stream: the handle's stream, after the work the caller queued on
     // the legacy default stream (its inputs and outputs are often written

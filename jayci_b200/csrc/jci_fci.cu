@@ -59,7 +59,10 @@ struct FciTables {
     uint32_t *sortB = nullptr;     // [Ib][f] beta singles sorted by target
     AbTables ab[2];                // fused product's entry lists, 8 / 16 column threads
     GroupTables grp[2];            // same-spin doubles by string groups, per spin
-    int *tc_status = nullptr;      // set by a product kernel whose bounded wait expired
+    // set by a product kernel whose bounded wait expired: host memory that the
+    // device writes, so that the host can look without waiting for it
+    volatile int *status = nullptr;
+    int *tc_status = nullptr;      // its device address
                                    // (tcgen05 product, row-shared panels)
     AbTables abk;                  // per-block lists of the column-blocked panel product
     void *tbufk[2] = {nullptr, nullptr};  // its per-CTA scratch blocks
@@ -121,10 +124,8 @@ jci_status fci_wait_status(jci_space *s) {
     const DeviceState *d = s->dev;
     if (d && d->emb) return embed_wait_status(d);
     if (!d || !d->fci || !d->fci->tc_status) return JCI_OK;
-    int flag = 0;
-    JCI_CUDA(cudaMemcpy(&flag, d->fci->tc_status, sizeof(int), cudaMemcpyDeviceToHost));
-    if (!flag) return JCI_OK;
-    JCI_CUDA(cudaMemset(d->fci->tc_status, 0, sizeof(int)));
+    if (!*d->fci->status) return JCI_OK;
+    *d->fci->status = 0;
     return JCI_ERR_TIMEOUT;
 }
 
@@ -139,7 +140,7 @@ void fci_free(DeviceState *d) {
         cudaFree(f->sbuf[s]);
     }
     cudaFree(f->sortB);
-    cudaFree(f->tc_status);
+    cudaFreeHost((void *)f->status);
     cudaFree(f->tbufk[0]);
     cudaFree(f->tbufk[1]);
     for (int p = 0; p < 2; p++) {
@@ -873,7 +874,7 @@ __global__ void __launch_bounds__(kMixThreads)
                            : wave_wait(&ctl->gemm_done[buf], (gen + 1) * ngi, ctl);
             if (!ok) {
                 atomicExch(&ctl->err, 1);
-                if (status) atomicExch(status, 1);
+                if (status) *(volatile int *)status = 1;
             }
             s_ok = ok;
         }
@@ -1442,8 +1443,10 @@ jci_status fci_prepare(jci_space *s) {
             JCI_CUDA(cudaMemcpy(f->sortB, so.data(), so.size() * sizeof(uint32_t),
                                 cudaMemcpyHostToDevice));
         }
-        JCI_CUDA(cudaMalloc(&f->tc_status, sizeof(int)));
-        JCI_CUDA(cudaMemset(f->tc_status, 0, sizeof(int)));
+        JCI_CUDA(cudaHostAlloc((void **)&f->status, sizeof(int),
+                               cudaHostAllocMapped | cudaHostAllocPortable));
+        *f->status = 0;
+        JCI_CUDA(cudaHostGetDevicePointer((void **)&f->tc_status, (void *)f->status, 0));
     }
     for (int sp = 0; sp < 2; sp++) {
         const SpinTables &t = d->t[sp];
@@ -1991,7 +1994,9 @@ static jci_status launch_ab(jci_space *s, const FciArgs<T> &fa, const T *v, T *o
             if ((r = launch_stream<T>(al, i8_stream_threads(f), v, o, st))) return r;
         }
         const I8Input<T> in{fa.sa, fa.fsA, fa.fpA, fa.m2, fa.skip};
-        return i8_launch<T>(f->i8, in, s->dev->device, v, o, f->tc_status, st);
+        const int expire = f->wave_expire;
+        f->wave_expire = 0;
+        return i8_launch<T>(f->i8, in, s->dev->device, v, o, f->tc_status, expire, st);
     }
     jci_status r = ab_tables(s, ab_table_tx(tx), st, &t);
     if (r) return r;

@@ -137,6 +137,7 @@ struct I8Args {
     const uint4 *lists;
     int lmax;                  // longest chunk list, in 16-byte units
     int npair;
+    int expire;                // test hook: CTA 0 never hands over its first chunk
     const int *skip;
 };
 
@@ -830,7 +831,12 @@ __global__ void __launch_bounds__(kIThreads, 1)
         // asked for, so that two are on their way
         bool pend = false;
         uint32_t prev = 0;
+        bool lose = a.expire && blockIdx.x == 0;
         auto hand = [&](uint32_t slot) {
+            if (lose) {
+                lose = false;
+                return;
+            }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             i8_arrive(bar_full + 8 * slot);
         };
@@ -1243,7 +1249,7 @@ __global__ void __launch_bounds__(kIThreads, 1)
         }
         failed = failed || !ok;
     }
-    if (failed && status) atomicExch(status, 1);
+    if (failed && status) *(volatile int *)status = 1;
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) {
@@ -1445,7 +1451,7 @@ jci_status i8_scratch(I8Tables *t, size_t w, size_t most) {
 // o += the alpha-single x beta-single part of H v.
 template <typename T>
 jci_status i8_launch(const I8Tables &t, const I8Input<T> &in, int device, const T *v, T *o,
-                     int *status, cudaStream_t st) {
+                     int *status, int expire, cudaStream_t st) {
     constexpr int p = sizeof(T) == 8 ? 0 : 1;
     unsigned char *base = (unsigned char *)t.scratch[p];
     if (!base || in.sa > 64) return JCI_ERR_STATE;
@@ -1470,6 +1476,7 @@ jci_status i8_launch(const I8Tables &t, const I8Input<T> &in, int device, const 
     a.vec = (size_t)t.nb * sizeof(T) % 16 == 0 && reinterpret_cast<uintptr_t>(v) % 16 == 0;
     a.lofs = t.lofs; a.lists = (const uint4 *)t.lists; a.lmax = t.lmax;
     a.npair = t.npair;
+    a.expire = expire;
     a.skip = in.skip;
     int nsm = 0;
     JCI_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
@@ -1485,8 +1492,8 @@ jci_status i8_launch(const I8Tables &t, const I8Input<T> &in, int device, const 
 }
 
 template jci_status i8_launch<double>(const I8Tables &, const I8Input<double> &, int,
-                                      const double *, double *, int *, cudaStream_t);
+                                      const double *, double *, int *, int, cudaStream_t);
 template jci_status i8_launch<float>(const I8Tables &, const I8Input<float> &, int, const float *,
-                                     float *, int *, cudaStream_t);
+                                     float *, int *, int, cudaStream_t);
 
 }  // namespace jci

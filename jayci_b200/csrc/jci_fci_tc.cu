@@ -442,7 +442,7 @@ __global__ void __launch_bounds__(NT, 1)
                 for (; issued[b] > 0 && mbar_wait(bar_mma0 + 8 * b, ph_mma[b]); issued[b]--)
                     ph_mma[b] ^= 1u;
             for (; lists > 0 && mbar_wait(bar_list, ph_list); lists--) ph_list ^= 1u;
-            if (status) atomicExch(status, 1);
+            if (status) *(volatile int *)status = 1;
         }
     }
     tc_fence_before();

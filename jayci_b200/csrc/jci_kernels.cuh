@@ -15,7 +15,8 @@ bool fci_supported(const jci_space *s);
 // device wait expired since the last call; synchronises with the device.
 jci_status fci_wait_status(jci_space *s);
 // Test hook: the next launch of the shared-panel product leaves the GEMM
-// items of its first rows undone, so that its gathers' waits expire.
+// items of its first rows undone, or that of the digit product keeps its first
+// chunk back, so that the waits for them expire.
 jci_status fci_arm_wait_expiry(jci_space *s);
 // Test hook: scratch buffers of more than this many bytes are refused.
 jci_status fci_limit_scratch(jci_space *s, size_t bytes);
@@ -100,7 +101,7 @@ size_t i8_smem(const I8Tables &t, int sa, size_t w);
 jci_status i8_scratch(I8Tables *t, size_t w, size_t most);
 template <typename T>
 jci_status i8_launch(const I8Tables &t, const I8Input<T> &in, int device, const T *v, T *o,
-                     int *status, cudaStream_t st);
+                     int *status, int expire, cudaStream_t st);
 
 // Same-spin doubles over groups of consecutive strings, jci_fci_group.cu.
 constexpr int kGroupRows = 16;
