@@ -124,7 +124,7 @@ bool embed_strings(const jci_space *s, long long n[2]) {
 
 // The full space and the string maps; false when there is none within the
 // limits or the device's free memory.
-static bool embed_build(jci_space *s) {
+static bool embed_try(jci_space *s) {
     DeviceState *d = s->dev;
     Embedding *e = d->emb;
     if (e->full) return true;
@@ -163,6 +163,16 @@ static bool embed_build(jci_space *s) {
         return false;
     }
     return true;
+}
+
+// Host memory that runs out is no usable full space either.
+static bool embed_build(jci_space *s) {
+    try {
+        return embed_try(s);
+    } catch (const std::bad_alloc &) {
+        embed_drop(s->dev->emb);
+        return false;
+    }
 }
 
 // Every sigma of the handle goes through the one pair of full vectors and the
