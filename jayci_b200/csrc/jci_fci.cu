@@ -2468,6 +2468,9 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
         int items = (f->nb + nt - 1) / nt;
         return !(nt > 32 * ((f->nb + 31) / 32) && nt > 128) && items <= 32;  // idle threads
     };
+    // In FP32 the digit product leaves half the rounding error of the 3xTF32 one
+    // (sigma's at FCI(12,12) 6e-8 and 1e-7): it may take 15% longer.
+    const float favour = prec ? 0.85f : 1.f;
     // the components of a plan are timed one by one; its best configuration is
     // timed end to end before choosing
     auto best_of = [&](auto fn) {
@@ -2540,7 +2543,10 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
     for (int tx : {8, 16, 32, 64, kI8Engine}) {
         if (only_split || !ab_plan_possible(s, tx, w, st)) continue;
         float ms = timeit([&] { return launch_ab<T>(s, ar, v, o, st, tx); });
-        if (ms < bab) { bab = ms; txab = tx; }
+        if (ms * (tx == kI8Engine ? favour : 1.f) < bab * (txab == kI8Engine ? favour : 1.f)) {
+            bab = ms;
+            txab = tx;
+        }
     }
     // best product behind the row kernel (modes 1, 2, 5) and behind the
     // stream passes (modes 3, 4)
@@ -2640,7 +2646,10 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
             if (!ab_plan_possible(s, tx, w, st)) continue;
             const float ms =
                 best_of([&] { return run_plan<T>(s, a, 5, kSplitSingles, tx, 1, v, o, st); });
-            if (ms < bestd) { bestd = ms; bdR = tx; }
+            if (ms * (tx == kI8Engine ? favour : 1.f) < bestd * (bdR == kI8Engine ? favour : 1.f)) {
+                bestd = ms;
+                bdR = tx;
+            }
         }
     }
     const int gmode = sab ? 7 : 6;
@@ -2671,14 +2680,19 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
     if (b1nt && best1 < best) { mode = b1mode; best = best1; }
     if (b3a && b3b && best3 < best) { mode = smode; best = best3; }
     if (best6 < best) { mode = gmode; best = best6; }
-    const bool split = bests < best;
+    const auto digits = [&]() {  // of the plan chosen so far
+        return (mode == 5 && b1mode == 5 && b1R == kI8Engine) ||
+               ((mode == 4 || mode == 7) && sR == kI8Engine);
+    };
+    const bool split = bests < 1e30f && bests * favour < best * (digits() ? favour : 1.f);
     if (split) {
         mode = 7;
         best = bests;
         b6s = kSplitSingles;
         b6i = bsB;
     }
-    const bool dense = bestd < best;
+    const bool dense = bestd < 1e30f && bestd * (bdR == kI8Engine ? favour : 1.f) <
+                                                                 best * (split || digits() ? favour : 1.f);
     if (dense) {
         mode = 5;
         best = bestd;

@@ -132,7 +132,7 @@ struct I8Args {
     const uint8_t *sl;         // [chunk][string][3][NS][16] digits of c, cut by column
     const T *cscale;           // [chunk * 48]
     const uint8_t *flags;      // [string][chunk] kIGraded | kISame, see k_i8_grade
-    const int *nstr, *strs;    // [2] numbers of plain and graded strings, [2][na] the strings
+    const int *nstr, *strs;    // numbers of plain and graded strings, [2][na] the strings
     const uint32_t *lofs;      // [chunk + 1] first 16-byte unit of each chunk's lists
     const uint4 *lists;
     int lmax;                  // longest chunk list, in 16-byte units
@@ -567,13 +567,13 @@ __global__ void __launch_bounds__(192)
     constexpr int NS = kDigits<T>;
     __shared__ int es[kIC];
     __shared__ int emax, emin;
-    __shared__ I8Mask ms[16];
+    __shared__ uint32_t ms[16][2][2];  // [row][near, some][24 columns | not finite << 31]
     const int c = blockIdx.x, nchunk = gridDim.x, tid = threadIdx.x;
     if (tid == 0) {
         emax = sizeof(T) == 8 ? kIEb : kIEbF;
         emin = 1 << 20;
     }
-    if (tid < 16) ms[tid].near = ms[tid].some = 0;
+    if (tid < 64) (&ms[0][0][0])[tid] = 0;
     __syncthreads();
     if (tid < kIC) {
         const int col = c * kIC + tid;
@@ -592,63 +592,125 @@ __global__ void __launch_bounds__(192)
     if (row < na) {
         T x[4];
         int eb[4];
-        unsigned long long near = 0, some = 0;
+        uint32_t near = 0, some = 0;
+        const int b0 = 4 * (q % 6);
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             const int e = es[4 * q + i];
             eb[i] = one || !e ? emax : e;
             x[i] = c0 + i < nb ? V[(long long)row * nb + c0 + i] : T(0);
             const uint32_t h = i8_high(x[i]);
-            if (x[i] != T(0)) some |= 1ull << (4 * q + i);  // (so is a NaN)
+            if (x[i] != T(0)) some |= 1u << (b0 + i);  // (so is a NaN)
             if (!i8_high_finite<T>(h)) {
                 x[i] = T(0);
-                some |= kINotFinite;
+                some |= 1u << 31;
             } else if ((int)(h >> (sizeof(T) == 8 ? 20 : 23)) >= eb[i] - kINear<T>) {
-                near |= 1ull << (4 * q + i);
+                near |= 1u << (b0 + i);
             }
         }
         i8_cut4<T, 16>(x, eb, sl + ((size_t)c * na + row) * NS * kIC + (q >> 2) * (NS * 16) +
                                   4 * (q & 3));
-        if (near) atomicOr(&ms[rl].near, near);
-        if (some) atomicOr(&ms[rl].some, some);
+        if (near) atomicOr(&ms[rl][0][q / 6], near);
+        if (some) atomicOr(&ms[rl][1][q / 6], some);
     }
     __syncthreads();
     if (tid < 16 && blockIdx.y * 16 + tid < na) {
-        if (one) ms[tid].near |= kISameBit;
-        masks[(size_t)(blockIdx.y * 16 + tid) * nchunk + c] = ms[tid];
+        const auto mask = [&](int k) {
+            return (unsigned long long)(ms[tid][k][0] & 0xffffffu) |
+                   (unsigned long long)(ms[tid][k][1] & 0xffffffu) << 24;
+        };
+        I8Mask m = {mask(0), mask(1)};
+        if (one) m.near |= kISameBit;
+        if ((ms[tid][1][0] | ms[tid][1][1]) >> 31) m.some |= kINotFinite;
+        masks[(size_t)(blockIdx.y * 16 + tid) * nchunk + c] = m;
     }
 }
 
 // The flags of a string's chunks from the masks of the rows that its singles
-// reach, and the string into the list of the plain or of the graded ones (in
-// any order: a string's sigma does not depend on it).  Bound by reading K
-// masks a chunk, from L2: 1 ms of 126 at FCI(16,16).
+// reach; the CTA that ends last then lists the plain and the graded strings in
+// their order (neighbours share most rows of c: FCI(16,16) 126.3 ms a sigma, 127.6
+// listed as they came in).  Bound by reading K masks a chunk, from L2: 1 ms of 126
+// at FCI(16,16).
 __global__ void __launch_bounds__(128)
     k_i8_grade(int na, int nchunk, int K, const uint32_t *__restrict__ fsA,
                const I8Mask *__restrict__ masks, uint8_t *__restrict__ flags,
-               int *__restrict__ nstr, int *__restrict__ strs, const int *skip) {
+               uint8_t *__restrict__ kind, int *__restrict__ nstr, int *__restrict__ strs,
+               const int *skip) {
     if (skip && *skip) return;
     __shared__ int rows[64];
-    const int Ia = blockIdx.x, tid = threadIdx.x;
+    __shared__ I8Mask part[4][32];
+    __shared__ int before[128], last;
+    const int Ia = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     if (tid < K) rows[tid] = (int)(fsA[(long long)tid * na + Ia] & 0x3fffffffu);
     __syncthreads();
     bool any = false;
-    for (int c = tid; c < nchunk; c += 128) {
-        unsigned long long near = 0, some = 0;
-#pragma unroll 8
-        for (int j = 0; j < K; j++) {
-            const I8Mask m = masks[(size_t)rows[j] * nchunk + c];
-            near |= m.near;
-            some |= m.some;
+    for (int c0 = 0; c0 < nchunk; c0 += 32) {  // a warp, every fourth row of 32 chunks
+        const int c = c0 + lane;
+        I8Mask m = {0, 0};
+        if (c < nchunk)
+#pragma unroll 4
+            for (int j = w; j < K; j += 4) {
+                const I8Mask x = masks[(size_t)rows[j] * nchunk + c];
+                m.near |= x.near;
+                m.some |= x.some;
+            }
+        part[w][lane] = m;
+        __syncthreads();
+        if (w == 0 && c < nchunk) {
+#pragma unroll
+            for (int k = 1; k < 4; k++) {
+                m.near |= part[k][lane].near;
+                m.some |= part[k][lane].some;
+            }
+            const bool graded = (m.some & ~m.near) != 0;
+            flags[(size_t)Ia * nchunk + c] =
+                (uint8_t)((graded ? kIGraded : 0) | (m.near & kISameBit ? kISame : 0));
+            any = any || graded;
         }
-        const bool graded = (some & ~near) != 0;
-        flags[(size_t)Ia * nchunk + c] =
-            (uint8_t)((graded ? kIGraded : 0) | (near & kISameBit ? kISame : 0));
-        any = any || graded;
+        __syncthreads();
     }
-    if (__syncthreads_or(any))
-        any = true;
-    if (tid == 0) strs[(any ? na : 0) + atomicAdd(nstr + (any ? 1 : 0), 1)] = Ia;
+    any = __syncthreads_or(any);
+    if (tid == 0) {
+        kind[Ia] = any;
+        __threadfence();
+        last = atomicAdd(nstr + 2, 1) == na - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    // thread t: 16 n strings from 16 n t on
+    const int n = ((na + 15) / 16 + 127) / 128, i0 = 16 * n * tid;
+    const auto words = [&](int v) {
+        uint4 x = make_uint4(0, 0, 0, 0);
+        if (i0 + 16 * v < na) x = __ldcg(reinterpret_cast<const uint4 *>(kind + i0 + 16 * v));
+        return x;
+    };
+    int count = 0;
+    for (int v = 0; v < n; v++) {
+        const uint4 x = words(v);  // (bytes behind the last string are zero)
+        count += __popc(x.x) + __popc(x.y) + __popc(x.z) + __popc(x.w);
+    }
+    before[tid] = count;
+    __syncthreads();
+    int g = 0;
+    for (int t = 0; t < tid; t++) g += before[t];
+    if (tid == 127) {
+        nstr[1] = g + count;
+        nstr[0] = na - g - count;
+    }
+    int p = min(i0, na) - g;
+    for (int v = 0; v < n; v++) {
+        const uint4 x = words(v);
+        const uint32_t q[4] = {x.x, x.y, x.z, x.w};
+        for (int k = 0; k < 16; k++) {
+            const int i = i0 + 16 * v + k;
+            if (i >= na) break;
+            if ((q[k >> 2] >> (8 * (k & 3))) & 1)
+                strs[na + g++] = i;
+            else
+                strs[p++] = i;
+        }
+    }
 }
 
 // The MMAs of one chunk that issuer I of NI takes: whole accumulators, so that
@@ -958,7 +1020,7 @@ __global__ void __launch_bounds__(kIThreads, 1)
                             reinterpret_cast<const unsigned char *>(a.cscale + (size_t)c * kIC) +
                                 16 * lane,
                             16);
-                    if (w == 0 && lane == 0) mode[r] = f & kISame ? kIOne : kIEach;
+                    if (GRADED && w == 0 && lane == 0) mode[r] = f & kISame ? kIOne : kIEach;
                     if (cutnext) fetch(c + 1);
                     __pipeline_commit();
                     if (pend) {
@@ -1159,14 +1221,23 @@ __global__ void __launch_bounds__(kIThreads, 1)
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             i8_sync_or<kIExt>(1, false);
             if (tid == 0) i8_arrive(bar_a);
+            const uint8_t *fl = a.flags + (size_t)Ia * nchunk;
+            uint32_t f = GRADED ? 0 : fl[0];
             for (int c = 0; c < nchunk; c++, g++) {
                 const uint32_t acc = NACC == 2 ? g & 1 : 0;
                 T *Ts = reinterpret_cast<T *>(smem + L.t + (g & 1) * L.tstride);
                 // the chunk's digits are there (which orders the loaders' scales and
                 // mode before the reads here), the gather of two chunks back is done,
                 // this chunk's MMAs are
-                ok = ok && i8_wait(bar_full + 8 * r, par);
-                const int md = mode[r];
+                int md;
+                if constexpr (GRADED) {
+                    ok = ok && i8_wait(bar_full + 8 * r, par);
+                    md = mode[r];
+                } else {  // known from the string's flags; FP64's integers need no scales here
+                    md = f & kISame ? kIOne : kIEach;
+                    f = c + 1 < nchunk ? fl[c + 1] : 0;
+                    if (md != kIOne) ok = ok && i8_wait(bar_full + 8 * r, par);
+                }
                 const bool bad = md == kIBad || !hfin, ints = NS == 7 && md == kIOne && hfin;
                 ok = ok && (g < 2 || i8_wait(bar_tfree + 8 * (g & 1), ((g >> 1) - 1) & 1));
                 ok = ok && i8_wait(bar_done + 8 * acc, (g / NACC) & 1);
@@ -1418,18 +1489,19 @@ size_t i8_smem(const I8Tables &t, int sa, size_t w) {
     return w == 8 ? i8_smem_bytes<double>(t, sa) : i8_smem_bytes<float>(t, sa);
 }
 
-// Scratch of one precision: column maxima and numbers of strings (zeroed before
-// each use), column scales, masks, flags, lists of strings, digits; the byte
+// Scratch of one precision: column maxima, numbers of strings and their kinds
+// (zeroed before each use), column scales, masks, flags, lists of strings, digits; the byte
 // offset of each.
 struct I8Scratch {
-    size_t nstr, scale, masks, flags, strs, sl, total;
+    size_t nstr, kind, scale, masks, flags, strs, sl, total;
 };
 static I8Scratch i8_scratch_layout(const I8Tables &t, size_t w, int ns) {
     auto up = [](size_t n) { return (n + 255) / 256 * 256; };
     const size_t blocks = (size_t)t.nchunk * t.na;
     I8Scratch l;
     l.nstr = up((size_t)t.nb * 4);
-    l.scale = l.nstr + up(2 * sizeof(int));
+    l.kind = l.nstr + up(3 * sizeof(int));
+    l.scale = l.kind + up((size_t)t.na + 15);
     l.masks = l.scale + up((size_t)t.nchunk * kIC * w);
     l.flags = l.masks + up(blocks * sizeof(I8Mask));
     l.strs = l.flags + up(blocks);
@@ -1466,8 +1538,8 @@ jci_status i8_launch(const I8Tables &t, const I8Input<T> &in, int device, const 
     k_i8_colmax<T><<<g1, 256, 0, st>>>(t.na, t.nb, v, mx, in.skip);
     dim3 g2(t.nchunk, (t.na + 15) / 16);
     k_i8_slice<T><<<g2, 192, 0, st>>>(t.na, t.nb, v, mx, sl, cscale, masks, in.skip);
-    k_i8_grade<<<t.na, 128, 0, st>>>(t.na, t.nchunk, in.sa, in.fsA, masks, flags, nstr, strs,
-                                     in.skip);
+    k_i8_grade<<<t.na, 128, 0, st>>>(t.na, t.nchunk, in.sa, in.fsA, masks, flags, base + l.kind,
+                                     nstr, strs, in.skip);
     I8Args<T> a;
     a.na = t.na; a.nb = t.nb; a.nchunk = t.nchunk; a.nrow = t.nrow; a.K = in.sa; a.KP = in.sa <= 32 ? 32 : 64;
     a.fsA = in.fsA; a.fpA = in.fpA; a.m2 = in.m2;
