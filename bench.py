@@ -33,6 +33,7 @@ from __future__ import annotations
 
 import argparse
 import json
+import math
 import os
 import statistics
 import sys
@@ -68,9 +69,9 @@ SIGMA_KERNELS = {0: 1, 1: 2, 2: 2, 3: 5, 4: 5, 5: 2, 6: 6, 7: 6}
 
 def sigma_kernels(mode, nt):
     """Kernels that a sigma of one vector launches at least (plan 7 with threads 1:
-    two transposes, two Coulomb passes, three of the product, two of each
+    two transposes, two Coulomb passes, five of the product, two of each
     spin's hole strings and column block)."""
-    return 11 if mode == 7 and nt == 1 else SIGMA_KERNELS[mode]
+    return 13 if mode == 7 and nt == 1 else SIGMA_KERNELS[mode]
 
 
 PLAN_NAMES = {0: "staged rows", 1: "row kernel, dense product through a global panel",
@@ -119,6 +120,23 @@ def sigma_plan_desc(mode, nt, R, B, ms=None):
     if ms is not None:
         d["autotuner_ms_per_vector"] = ms
     return d
+
+
+def sigma_flops(sp):
+    """FP64 operations that one sigma of a one-group space cannot do without: the
+    alpha x beta part as a product per alpha string (its singles x the pairs that
+    the beta strings read, or every double replacement where that is less), and a
+    multiply-add for every same-spin replacement."""
+    n, oa, ob = sp.norb, sp.na, sp.nb
+    sa, sb = oa * (n - oa), ob * (n - ob)
+    same = sum(o * (n - o) + math.comb(o, 2) * math.comb(n - o, 2) for o in (oa, ob))
+    return 2.0 * sp.ndets * (min(sa * sb, sa * (1 + ob + sb)) + same)
+
+
+def fp64_peak(torch):
+    """TFLOP/s of 64 multiply-adds a clock and SM at the maximum SM clock (1 965 MHz)."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    return sms * 64 * 2 * 1.965e9 / 1e12
 
 
 def max_over_ranks(dist, values, device):
@@ -507,7 +525,7 @@ def run_gpu(a):
 
         import torch.distributed as dist
         dist.init_process_group("nccl", timeout=datetime.timedelta(seconds=300))
-    (geo, nroots, s_exc, d_exc) = WORKLOADS[a.workload]
+    (geo, nroots, _, _) = WORKLOADS[a.workload]
     ints = workload_integrals(a.workload)
     m1, m2 = ints.packed()
     setup = {}
@@ -600,21 +618,25 @@ def run_gpu(a):
     e2e = replica_rate(world, N * nvec * a.steps, e2e_s) / 1e9
     del hv, hs, hvn, hsn
 
-    # roofline of the sigma kernel (row-stream algorithmic bytes per vector)
-    w = 8
-    bytes_per_launch = w * N * (2 + s_exc + d_exc)
+    # roofline of a sigma: the FP64 operations that it cannot do without
     avg_launch_s = statistics.mean(launches) / 1e3
-    peak, peak_kind = measured_peaks()
-    achieved = bytes_per_launch / avg_launch_s / 1e9
+    flops, peak = sigma_flops(sp), fp64_peak(torch)
+    achieved = flops / avg_launch_s / 1e12
+    hbm_peak, hbm_kind = measured_peaks()
     mode, nt, R, B, tms = sp.sigma_tuning(jb.FP64)
     tune32 = sp.sigma_tuning(jb.FP32)
     prof = committed_profile(a.workload, mode, B, R, nt) or {}
-    roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-            "frac": achieved / peak, "traffic": prof.get("dram_bytes_per_launch"),
-            "algorithmic_bytes_per_launch": bytes_per_launch, "peak_source": peak_kind,
+    roof = {"bound": "fp64", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
+            "frac": achieved / peak, "flops_per_launch": flops,
+            "peak_source": "64 FP64 multiply-adds a clock and SM (measured, FMA and tensor pipe) "
+                           "at the maximum SM clock",
             "kernel_ms_per_launch": avg_launch_s * 1e3,
-            "model": "row-stream bytes B = 8 N (2 + s + d) per vector: each sigma row reads "
-                     "its own C row and one C row per alpha single and double"}
+            "model": "2 N (alpha x beta part + same-spin replacements) per vector: per alpha "
+                     "single one product row for every pair that a beta string reads, one "
+                     "multiply-add per same-spin replacement; c and sigma once are "
+                     f"{16 * N / 1e9:.3f} GB",
+            "traffic": prof.get("dram_bytes_per_launch"), "hbm_peak_gb_per_s": hbm_peak,
+            "hbm_peak_source": hbm_kind}
     for k in ("dram_gb_per_s", "l2_bytes_per_launch", "dominant_kernel", "limiter", "summary"):
         if k in prof:
             roof[k] = prof[k]

@@ -229,7 +229,9 @@ jci_status jci_sigma_device_noalloc(jci_space *s, const void *v, void *sigma,
  * chunks: FP64 mma.sync in FP64, 3xTF32 in FP32), or in FP32 32 / 64 (the
  * tcgen05 engine, 32- / 64-column chunks), or 128 (8-bit digit products on
  * the tcgen05 integer tensor cores, 48-column chunks, FP64 and FP32; at most
- * 64 alpha singles and 127 pairs)), `batch` (modes 1, 2, 5: alpha strings
+ * 64 alpha singles and 127 pairs; as accurate as the floating engines in the
+ * elements of v that H connects to an element of sigma, and in the integrals to
+ * 2^-55 (FP64) or 2^-31 (FP32) of the largest one)), `batch` (modes 1, 2, 5: alpha strings
  * per CTA of the row kernel; modes 3-4: threads per CTA of the beta pass; modes 6-7: the
  * group kernel variant, 1 or 2 columns per thread, or 3, 4: the group's
  * excitation targets split over 4 warps with 2 or 1 columns per lane, or

@@ -14,8 +14,8 @@
 // in different orders; a caller that needs the same bits in every process
 // reads the route and pins it (embed_route, embed_set_route).
 // Measured: 12 electrons in 16 orbitals (2 DOCC, 10 active, 4 virtual,
-// excitation level 2; 13.0 of 64.1 million determinants) FP64 215 -> 45.3 ms,
-// FP32 188 -> 32.2; 11 electrons in 15 orbitals (2 DOCC, 9 active; 3.2 of 15.0
+// excitation level 2; 13.0 of 64.1 million determinants) FP64 215 -> 53.3 ms,
+// FP32 188 -> 34.4; 11 electrons in 15 orbitals (2 DOCC, 9 active; 3.2 of 15.0
 // million) FP64 40 -> 10.0 ms; 11 in 12 (1 DOCC, 7 active; 0.12 of 0.73
 // million) 0.73 -> 0.48 ms.
 #include <cuda_runtime.h>

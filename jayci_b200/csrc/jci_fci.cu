@@ -2637,7 +2637,7 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
     // mode 5 with the same-spin part as dense products, end to end.  Measured
     // (us, best of the other plans -> this one): N electrons in N orbitals
     // FP64 N = 8 32 -> 24, 9 38 -> 24, 10 64 -> 40, 11 163 -> 130, 12 549 -> 488;
-    // FP32 9 37 -> 24, 10 57 -> 36, 11 142 -> 118, 12 398 -> 385; 8 in 13
+    // FP32 9 37 -> 24, 10 57 -> 36, 11 142 -> 118, 12 438 -> 408; 8 in 13
     // orbitals FP64 379 -> 335.  At N = 13 (1 716 strings) the lists win.
     float bestd = 1e30f;
     int bdR = 0;
