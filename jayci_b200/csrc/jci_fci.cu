@@ -2385,10 +2385,11 @@ static jci_status run_plan(jci_space *s, FciArgs<T> a, int mode, int nt, int R, 
 }
 
 // The vector that plans are timed on: pseudo-random elements that shrink by
-// 10^0.4 for every electron above the lowest orbitals, over some six decades
-// at FCI(16,16).  The digit product's time depends on how its vector is graded
-// (FCI(14,14) FP64 7.2 ms a sigma for a random one, 8.8 for a CI vector); a
-// solve's vectors look like this one.
+// 10^0.25 for every electron above the lowest orbitals, over four decades at
+// FCI(16,16).  The digit product's time depends on how its vector is graded
+// (13 electrons in 13 orbitals, FP64: 1.78 ms a sigma for a random one, 1.93 for
+// this one, 2.25 for 10^0.8 an electron); zeros and random vectors are its best
+// case, a solve's vectors lie between.
 template <typename T>
 __global__ void k_tune_vector(int na, int nb, int nela, int nelb,
                               const uint64_t *__restrict__ oa, const uint64_t *__restrict__ ob,
@@ -2400,7 +2401,7 @@ __global__ void k_tune_vector(int na, int nb, int nela, int nelb,
     x = (x ^ (x >> 16)) * 2246822519u;
     x ^= x >> 13;
     const float u = (float)(int32_t)x * (1.f / 2147483648.f);
-    v[i] = (T)(u * exp10f(-0.4f * lev));
+    v[i] = (T)(u * exp10f(-0.25f * lev));
 }
 
 // Pick the plan for this space by timing the admissible candidates on
@@ -2469,8 +2470,9 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
         return !(nt > 32 * ((f->nb + 31) / 32) && nt > 128) && items <= 32;  // idle threads
     };
     // In FP32 the digit product leaves half the rounding error of the 3xTF32 one
-    // (sigma's at FCI(12,12) 6e-8 and 1e-7): it may take 15% longer.
-    const float favour = prec ? 0.85f : 1.f;
+    // (sigma's at FCI(12,12) 5e-8 and 1e-7): where the two are level within 5%, it
+    // is taken (FCI(12,12) 402 and 408 us; 10 in 12, 15 us slower, it is not).
+    const float favour = prec ? 0.95f : 1.f;
     // the components of a plan are timed one by one; its best configuration is
     // timed end to end before choosing
     auto best_of = [&](auto fn) {
@@ -2500,8 +2502,8 @@ static jci_status autotune(jci_space *s, FciArgs<T> a, cudaStream_t st) {
         }
     }
     // From 2^21 determinants on no other plan beats it, and timing those would
-    // take half a minute at the largest.  Measured on the graded vector (ms,
-    // split / best of the others; electrons in orbitals, alpha singles): 13 in 13
+    // take half a minute at the largest.  Measured on a vector graded by 10^0.4 an
+    // electron, against the split plan (ms, split / best of the others; electrons in orbitals, alpha singles): 13 in 13
     // (42) FP64 2.21 / 2.21, FP32 1.23 / 1.45; 10 in 14 (45) 3.10 / 3.27, 1.67 /
     // 1.95; 9 in 15 (50) 3.34 / 3.66, 1.90 / 2.25; 12 in 14 (48) 7.09 / 7.92,
     // 4.06 / 4.76; 14 in 14 (49) 9.31 / 10.8, 4.98 / 5.96; 10 in 16 (55) 15.0 /
